@@ -210,6 +210,43 @@ __device__ __forceinline__ const double* chain_off<double>(const mcv_chain& ch,
 }
 
 // ------------------------------------------------------------ math
+// FP32 quotients and roots of lengths, speeds and times.  The kernels keep
+// denormals (no --ftz), and with that the compiler wraps every approximate
+// reciprocal and root in range tests and rescalings: 2-4 instructions each,
+// a quarter of the guide chain's.  No quantity these are applied to is
+// denormal unless it is 0 or lost already (a speed or length under 1e-38, a
+// quotient whose reciprocal overflows), so here they are the bare hardware
+// operation, which gives the same bits on every other argument.
+__device__ __forceinline__ float f_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float f_sqrt(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float f_rsqrt(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float f_div(float a, float b) {
+  return __fmul_rn(a, f_rcp(b));
+}
+__device__ __forceinline__ double f_div(double a, double b) { return a / b; }
+
+// a / b from r = 1 / b (correctly rounded): one residual correction of a r
+// gives the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34,
+// 1990), so several quotients by one divisor cost three FP64 operations each
+// instead of a division's ten, with the division's result.  Finite operands
+// and quotients in the normal range.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q = __dmul_rn(a, r);
+  return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+
 __device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double m_sqrt(double x) { return sqrt(x); }
 // square root of a uniform: the reference applies math.sqrt to the float32

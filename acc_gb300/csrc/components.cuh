@@ -17,7 +17,17 @@ namespace mcv {
 // Source_simple.propagate (acc/components/sources/source_simple.py:114-162)
 // with randvec_target_rect (:17-42) for the target on the z axis, where the
 // two normalised perpendiculars are (-1,0,0) and (0,-1,0).
-template <typename R, typename Rng>
+//
+// kWave: the wave kernels' FP32 form (wave.cuh), on the bare hardware
+// reciprocal and roots and with the roundings of its sums spelled out: the
+// compiler's choice of which product to contract into a multiply-add depends
+// on the code around an inlined call, and every kernel has to follow the same
+// neutron.  (The multiple-scattering kernel ran 2.4% slower with it.)
+__device__ __forceinline__ float sum_squares(float a, float b, float c) {
+  return fmaf(c, c, fmaf(a, a, __fmul_rn(b, b)));
+}
+
+template <typename R, bool kWave = false, typename Rng>
 __device__ __forceinline__ void source_simple(Neutron<R>& n, Rng& rng,
                                               const mcv_component& c) {
   const R width = prm<R>(c, 0), height = prm<R>(c, 1), radius = prm<R>(c, 2);
@@ -39,31 +49,42 @@ __device__ __forceinline__ void source_simple(Neutron<R>& n, Rng& rng,
   }
   R tdx = xw * (r3 * 2 - 1) / R(2.0);
   R tdy = yh * (r4 * 2 - 1) / R(2.0);
-  R dist2 = m_sqrt(tdx * tdx + tdy * tdy + dist * dist);
-  R solidangle = (xw * yh * dist) / (dist2 * dist2 * dist2);
+  R solidangle;
+  constexpr bool kBare = kWave && sizeof(R) == 4;
+  if constexpr (kBare) {
+    R dist2 = f_sqrt(sum_squares(tdx, tdy, dist));
+    solidangle = f_div(xw * yh * dist, dist2 * dist2 * dist2);
+  } else {
+    R dist2 = m_sqrt(tdx * tdx + tdy * tdy + dist * dist);
+    solidangle = (xw * yh * dist) / (dist2 * dist2 * dist2);
+  }
   R dx = -tdx - x, dy = -tdy - y;
   R v;
   if (c.ip[1]) {
     R L = Lambda0 + dLambda * (r5 * 2 - 1);
-    v = R(kK2V) * (R(2 * kPi) / L);
+    if constexpr (kBare) v = R(kK2V) * f_div(R(2 * kPi), L);
+    else v = R(kK2V) * (R(2 * kPi) / L);
   } else {
     R E = E0 + dE * (r5 * 2 - 1);
-    v = R(kSE2V) * m_sqrt(E);
+    if constexpr (kBare) v = R(kSE2V) * f_sqrt(E);
+    else v = R(kSE2V) * m_sqrt(E);
   }
   n.x = x;
   n.y = y;
   n.z = R(0);
   if constexpr (sizeof(R) == 4) {
-    R inv = m_rsqrt(dx * dx + dy * dy + dist * dist);
+    R inv;
+    if constexpr (kBare) inv = f_rsqrt(sum_squares(dx, dy, dist));
+    else inv = m_rsqrt(dx * dx + dy * dy + dist * dist);
     R vs = v * inv;
     n.vx = vs * dx;
     n.vy = vs * dy;
     n.vz = vs * dist;
   } else {
-    R dist1 = m_sqrt(dx * dx + dy * dy + dist * dist);
-    n.vx = v * dx / dist1;
-    n.vy = v * dy / dist1;
-    n.vz = v * dist / dist1;
+    R dist1 = m_sqrt(dx * dx + dy * dy + dist * dist), inv = 1.0 / dist1;
+    n.vx = div_by(v * dx, dist1, inv);
+    n.vy = div_by(v * dy, dist1, inv);
+    n.vz = div_by(v * dist, dist1, inv);
   }
   n.sx = R(0);
   n.sy = R(0);
@@ -409,11 +430,13 @@ __device__ __forceinline__ float reflectivity(float Q, float R0, float Qc,
 // writes back at line 160.
 
 // false when the neutron is absorbed at the opening (only p changes then)
-template <typename R>
+template <typename R, bool kWave = false>
 __device__ __forceinline__ bool guide_enter(Neutron<R>& n,
                                             const mcv_component& c) {
   const R hw1 = prm<R>(c, 2), hh1 = prm<R>(c, 3);
-  R dt = -n.z / n.vz;
+  R dt;
+  if constexpr (kWave) dt = f_div(-n.z, n.vz);
+  else dt = -n.z / n.vz;
   R x = n.x + n.vx * dt;
   R y = n.y + n.vy * dt;
   if (x <= -hw1 || x >= hw1 || y <= -hh1 || y >= hh1) {
@@ -427,13 +450,41 @@ __device__ __forceinline__ bool guide_enter(Neutron<R>& n,
   return true;
 }
 
+// What an FP64 bounce divides by, with its reciprocals (div_by): the length
+// |n| and |n|^2 of the side (x) and top (y) mirrors' normals (l, slope), and
+// the edge width W.  A kernel that keeps them in shared memory forms them
+// once a block; without them (nullptr) a bounce divides.
+struct GuideInv {
+  double n[2], rn[2], n2[2], rn2[2], rw;
+};
+__device__ __forceinline__ GuideInv guide_inv(const mcv_component& c) {
+  const double l = c.dp[4];
+  GuideInv g;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    g.n2[k] = l * l + c.dp[k] * c.dp[k];
+    g.n[k] = sqrt(g.n2[k]);
+    g.rn[k] = 1.0 / g.n[k];
+    g.rn2[k] = 1.0 / g.n2[k];
+  }
+  g.rw = 1.0 / c.dp[9];
+  return g;
+}
+
 // One pass of the bounce loop in FP32, without branches: lanes of a warp
 // reach the same bounce with different walls ahead, so every candidate
 // time is formed and the earliest is kept by selects (same comparison order
 // as the reference, guide.py:100-123); the reflection and the reflectivity
 // are selected the same way.  Division by a zero normal product gives an
 // infinity that the "approaching" test never selects.
-template <typename Trk>
+//
+// kWave: the form of the wave kernels (wave.cuh), with every rounding spelled
+// out: inlined into their two loops, the compiler contracted different
+// products into multiply-adds, and their neutrons drifted apart by an ulp
+// (3 bin changes in the PSD of 1e8 guide-chain neutrons).  The times come
+// from normal products rounded at every step, the reflection from one
+// contracted product.
+template <bool kWave, typename Trk>
 __device__ __forceinline__ bool guide_bounce_fp32(Neutron<float>& n,
                                                   const mcv_component& c,
                                                   Trk& trk) {
@@ -441,14 +492,32 @@ __device__ __forceinline__ bool guide_bounce_fp32(Neutron<float>& n,
               hw1 = prm<float>(c, 2), hh1 = prm<float>(c, 3),
               l = prm<float>(c, 4);
   const float x = n.x, y = n.y, z = n.z, vx = n.vx, vy = n.vy, vz = n.vz;
-  const float av = l * vx, bv = ww * vz, ah = l * vy, bh = hh * vz;
-  const float vn1 = bv + av, vn2 = bv - av, vn3 = bh + ah, vn4 = bh - ah;
-  const float cv1 = -hw1 * l - z * ww, cv2 = x * l;
-  const float ch1 = -hh1 * l - z * hh, ch2 = y * l;
-  float t1 = (l - z) / vz;
+  float t1, s1, s2, s3, s4, vn1, vn2, vn3, vn4, ax = 0.f, ay = 0.f;
+  if constexpr (kWave) {
+    ax = __fmul_rn(l, vx);
+    ay = __fmul_rn(l, vy);
+    const float bx = __fmul_rn(ww, vz), by = __fmul_rn(hh, vz);
+    vn1 = __fadd_rn(bx, ax);
+    vn2 = __fsub_rn(bx, ax);
+    vn3 = __fadd_rn(by, ay);
+    vn4 = __fsub_rn(by, ay);
+    const float cx = fmaf(-hw1, l, -__fmul_rn(z, ww));
+    const float cy = fmaf(-hh1, l, -__fmul_rn(z, hh));
+    t1 = f_div(l - z, vz);
+    s1 = f_div(fmaf(-x, l, cx), vn1);
+    s2 = f_div(fmaf(x, l, cx), vn2);
+    s3 = f_div(fmaf(-y, l, cy), vn3);
+    s4 = f_div(fmaf(y, l, cy), vn4);
+  } else {
+    const float av = l * vx, bv = ww * vz, ah = l * vy, bh = hh * vz;
+    vn1 = bv + av, vn2 = bv - av, vn3 = bh + ah, vn4 = bh - ah;
+    const float cv1 = -hw1 * l - z * ww, cv2 = x * l;
+    const float ch1 = -hh1 * l - z * hh, ch2 = y * l;
+    t1 = (l - z) / vz;
+    s1 = (cv1 - cv2) / vn1, s2 = (cv1 + cv2) / vn2;
+    s3 = (ch1 - ch2) / vn3, s4 = (ch1 + ch2) / vn4;
+  }
   int i = 0;
-  const float s1 = (cv1 - cv2) / vn1, s2 = (cv1 + cv2) / vn2;
-  const float s3 = (ch1 - ch2) / vn3, s4 = (ch1 + ch2) / vn4;
   if (vn1 < 0.f && s1 < t1) { t1 = s1; i = 1; }
   if (vn2 < 0.f && s2 < t1) { t1 = s2; i = 2; }
   if (vn3 < 0.f && s3 < t1) { t1 = s3; i = 3; }
@@ -459,11 +528,18 @@ __device__ __forceinline__ bool guide_bounce_fp32(Neutron<float>& n,
   n.z = fmaf(vz, t1, z);
   n.t.add(t1);
   const bool xw = i <= 2;
-  const float vdn = i == 1 ? vn1 : i == 2 ? vn2 : i == 3 ? vn3 : vn4;
   const float lw = xw ? ww : hh;
+  float vdn;
+  if constexpr (kWave) {
+    const float a = xw ? ax : ay;
+    vdn = fmaf(lw, vz, i == 1 || i == 3 ? a : -a);
+  } else {
+    vdn = i == 1 ? vn1 : i == 2 ? vn2 : i == 3 ? vn3 : vn4;
+  }
   // mirror parallel to z: the reflection flips one component exactly,
   // q = 2 V2K |v_perp|; inclined mirror: v -= 2 (v.n) n / |n|^2
-  const float rn = rsqrtf(fmaf(l, l, lw * lw));
+  const float rn = kWave ? f_rsqrt(fmaf(l, l, lw * lw))
+                         : rsqrtf(fmaf(l, l, lw * lw));
   const float d = 2.f * vdn * (rn * rn);
   const float sg = (i == 1 || i == 3) ? -1.f : 1.f;
   const bool flat = lw == 0.f;
@@ -480,86 +556,110 @@ __device__ __forceinline__ bool guide_bounce_fp32(Neutron<float>& n,
   trk.reflect(q, R0, Qc, alpha, m, W);
   // calc_reflectivity (_guide_utils.py:6-23) with (1 - tanh x) / 2 =
   // 1 / (1 + e^(2x)), evaluated for every lane and selected
-  const float tmp = (q - m * Qc) / W;
-  const float edge = R0 * (1.f - alpha * (q - Qc)) / (1.f + expf(2.f * tmp));
+  float edge, tmp;
+  if constexpr (kWave) {
+    tmp = f_div(fmaf(-m, Qc, q), W);
+    edge = f_div(__fmul_rn(R0, fmaf(-alpha, q - Qc, 1.f)),
+                 1.f + expf(2.f * tmp));
+  } else {
+    tmp = (q - m * Qc) / W;
+    edge = R0 * (1.f - alpha * (q - Qc)) / (1.f + expf(2.f * tmp));
+  }
   const float refl = q > Qc ? (tmp < 10.f ? edge : 0.f) : R0;
   n.p *= refl;
   return n.p <= 0.f;
 }
 
-// One pass of the bounce loop in FP64, in the reference's operation order.
+// One pass of the bounce loop in FP64, rounded as the reference's
+// (guide.py:100-159).  The FP64 pipe bounds it (2 lanes a clock and SM), and
+// a division or root is some ten operations of it, so the walls' times are
+// compared as fractions (cross-multiplied, denominators made positive) and
+// only the earliest is divided out; the two side walls (and the two
+// horizontal ones) share their instructions, since a neutron approaches both
+// of a pair only in a strongly converging guide; and the mirror's constants
+// divide through their reciprocals.
 template <typename Trk>
 __device__ __forceinline__ bool guide_bounce_fp64(Neutron<double>& n,
                                                   const mcv_component& c,
-                                                  Trk& trk) {
+                                                  Trk& trk,
+                                                  const GuideInv* inv) {
   const double ww = c.dp[0], hh = c.dp[1], hw1 = c.dp[2], hh1 = c.dp[3],
                l = c.dp[4];
-  double x = n.x, y = n.y, z = n.z, vx = n.vx, vy = n.vy, vz = n.vz;
-  double av = l * vx, bv = ww * vz, ah = l * vy, bh = hh * vz;
-  double vdotn_v1 = bv + av, vdotn_v2 = bv - av;
-  double vdotn_h1 = bh + ah, vdotn_h2 = bh - ah;
-  double cv1 = -hw1 * l - z * ww, cv2 = x * l;
-  double ch1 = -hh1 * l - z * hh, ch2 = y * l;
-  double t1 = (l - z) / vz, t2;
+  const double x = n.x, y = n.y, z = n.z, vx = n.vx, vy = n.vy, vz = n.vz;
+  const double av = l * vx, bv = ww * vz, ah = l * vy, bh = hh * vz;
+  const double vn1 = bv + av, vn2 = bv - av, vn3 = bh + ah, vn4 = bh - ah;
+  const double cv1 = hw1 * l + z * ww, cv2 = x * l;
+  const double ch1 = hh1 * l + z * hh, ch2 = y * l;
+  // the earliest time so far, num / den with den >= 0 (0: at infinity)
+  double num = vz < 0 ? z - l : l - z, den = m_fabs(vz), vdn = 0;
   int i = 0;
-  if (vdotn_v1 < 0) {
-    t2 = (cv1 - cv2) / vdotn_v1;
-    if (t2 < t1) { t1 = t2; i = 1; }
+  auto ahead = [&](double a, double v, int wall) {
+    // the wall's time is a / (-v), v < 0
+    if (a * den < num * -v) {
+      num = a;
+      den = -v;
+      vdn = v;
+      i = wall;
+    }
+  };
+  if (vn1 < 0 || vn2 < 0) {
+    const bool one = vn1 < 0;
+    ahead(one ? cv1 + cv2 : cv1 - cv2, one ? vn1 : vn2, one ? 1 : 2);
+    if (one && vn2 < 0) ahead(cv1 - cv2, vn2, 2);
   }
-  if (vdotn_v2 < 0) {
-    t2 = (cv1 + cv2) / vdotn_v2;
-    if (t2 < t1) { t1 = t2; i = 2; }
-  }
-  if (vdotn_h1 < 0) {
-    t2 = (ch1 - ch2) / vdotn_h1;
-    if (t2 < t1) { t1 = t2; i = 3; }
-  }
-  if (vdotn_h2 < 0) {
-    t2 = (ch1 + ch2) / vdotn_h2;
-    if (t2 < t1) { t1 = t2; i = 4; }
+  if (vn3 < 0 || vn4 < 0) {
+    const bool one = vn3 < 0;
+    ahead(one ? ch1 + ch2 : ch1 - ch2, one ? vn3 : vn4, one ? 3 : 4);
+    if (one && vn4 < 0) ahead(ch1 - ch2, vn4, 4);
   }
   if (i == 0) return true;  // the neutron left the guide
+  const double t1 = num / den;
   n.x = x + vx * t1;
   n.y = y + vy * t1;
   n.z = z + vz * t1;
   n.t.add(t1);
-  double vdn = (i == 1) ? vdotn_v1 : (i == 2) ? vdotn_v2 : (i == 3) ? vdotn_h1
-                                                                   : vdotn_h2;
-  double lw = (i <= 2) ? ww : hh;  // the mirror's slope term
-  double nlen2 = l * l + lw * lw;
-  double q = kV2K * (-2) * vdn / sqrt(nlen2);
-  double d = 2 * vdn / nlen2;
-  if (i == 1) {
-    n.vx = vx - d * l;
-    n.vz = vz - d * ww;
-  } else if (i == 2) {
-    n.vx = vx + d * l;
-    n.vz = vz - d * ww;
-  } else if (i == 3) {
-    n.vy = vy - d * l;
-    n.vz = vz - d * hh;
+  const bool side = i <= 2;
+  const double lw = side ? ww : hh;  // the mirror's slope term
+  double q = kV2K * (-2) * vdn, d = 2 * vdn;
+  if (inv) {
+    const int w = side ? 0 : 1;
+    q = div_by(q, inv->n[w], inv->rn[w]);
+    d = div_by(d, inv->n2[w], inv->rn2[w]);
   } else {
-    n.vy = vy + d * l;
-    n.vz = vz - d * hh;
+    const double nlen2 = l * l + lw * lw;
+    q = q / sqrt(nlen2);
+    d = d / nlen2;
   }
+  const double turn = (i == 1 || i == 3 ? -d : d) * l;
+  const double vp = (side ? vx : vy) + turn;
+  n.vx = side ? vp : vx;
+  n.vy = side ? vy : vp;
+  n.vz = vz - d * lw;
   const double R0 = c.dp[5], Qc = c.dp[6], alpha = c.dp[7], m = c.dp[8],
                W = c.dp[9];
   trk.reflect(q, R0, Qc, alpha, m, W);
-  n.p *= reflectivity(q, R0, Qc, alpha, m, W);
+  // calc_reflectivity (_guide_utils.py:6-23)
+  double refl = R0;
+  if (q > Qc) {
+    const double e = q - m * Qc, tmp = inv ? div_by(e, W, inv->rw) : e / W;
+    refl = 0;
+    if (tmp < 10) refl = R0 * ((1 - tanh(tmp)) * (1 - alpha * (q - Qc)) / 2);
+  }
+  n.p *= refl;
   return n.p <= 0;
 }
 
 // one pass of the bounce loop; true when the neutron has left the guide
 // (it stays at its last reflection point, guide.py:122-123) or its weight
 // is gone
-template <typename R, typename Trk>
+template <typename R, bool kWave = false, typename Trk>
 __device__ __forceinline__ bool guide_bounce(Neutron<R>& n,
-                                             const mcv_component& c,
-                                             Trk& trk) {
+                                             const mcv_component& c, Trk& trk,
+                                             const GuideInv* inv = nullptr) {
   if constexpr (sizeof(R) == 4)
-    return guide_bounce_fp32(n, c, trk);
+    return guide_bounce_fp32<kWave>(n, c, trk);
   else
-    return guide_bounce_fp64(n, c, trk);
+    return guide_bounce_fp64(n, c, trk, inv);
 }
 
 // The whole guide; returns 1 when the bounce loop ran out of its

@@ -510,12 +510,13 @@ bool host_is_monitor(const mcv_component& c) {
   }
 }
 
-// The FP32 fused run uses path regeneration when asked to, or by default
-// when the chain has a guide (whose bounce count varies from neutron to
-// neutron) or a long segmented guide (one taking quiet blocks, ip[1] > 0:
+// Path regeneration of a kX chain (regen_kernel, FP32): when asked to, or by
+// default when the chain has a guide (whose bounce count varies from neutron
+// to neutron) or a long segmented guide (one taking quiet blocks, ip[1] > 0:
 // a neutron may die in its first segment or fly through all of them; VERDI
 // 5.68e8 n/s against 5.32e8); chains without one have near-uniform paths.
 bool use_regen(const mcv_chain* ch, const mcv_launch* launch) {
+  if (!is_exotic(ch)) return false;
   if (has_hms(ch)) return false;  // the fan-out runs in the thread kernel
   if (launch && launch->variant == 1) return false;
   if (launch && (launch->variant == 2 || launch->variant == 3)) return true;
@@ -527,15 +528,47 @@ bool use_regen(const mcv_chain* ch, const mcv_launch* launch) {
   return false;
 }
 
-// Shared memory of the regeneration kernel's tail queue for blocks of
+int last_guide_of(const mcv_chain* ch) {
+  int last = -1;
+  for (int k = 0; k < ch->ncomp; ++k)
+    if (ch->comp[k].opcode == MCV_OP_GUIDE) last = k;
+  return last;
+}
+
+// Chains with a guide run the wave kernels (wave.cuh) unless the launch asks
+// for the thread kernel (variant 1): neutrons differ in their number of
+// reflections.  Without a guide there is nothing to regroup by.
+bool use_wave(const mcv_chain* ch, const mcv_launch* launch) {
+  return !is_exotic(ch) && last_guide_of(ch) >= 0 &&
+         !(launch && launch->variant == 1);
+}
+
+// Neutrons that wait for the components after the last guide before those
+// run: a warp of them (variant 3: none).
+int wave_tail_min(const mcv_launch* launch) {
+  return launch && launch->variant == 3 ? 1 : 32;
+}
+
+template <typename R>
+void launch_wave(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
+                 uint64_t first, uint64_t seed, const mcv_launch* launch,
+                 cudaStream_t s) {
+  int blocks, threads;
+  const int tw = sizeof(R) == 4 ? smem_tally_words(chain) : 0;
+  launch_shape(
+      ctx, [tw](int t) { return Launchers<R>::occupancy_wave(t, tw); },
+      ncount, launch, &blocks, &threads);
+  Launchers<R>::wave(blocks, threads, wave_tail_min(launch), tw, s, *chain,
+                     ncount, first, seed, ctx->d_status);
+}
+
+// Shared memory of the regeneration kernels' tail queue for blocks of
 // `threads`: one queue per warp when components follow the chain's last
 // guide (variant 3 runs without it).
 size_t regen_tail_bytes(const mcv_chain* ch, const mcv_launch* launch,
                         int threads) {
   if (launch && launch->variant == 3) return 0;
-  int last = -1;
-  for (int k = 0; k < ch->ncomp; ++k)
-    if (ch->comp[k].opcode == MCV_OP_GUIDE) last = k;
+  const int last = last_guide_of(ch);
   if (last < 0 || last + 1 >= ch->ncomp) return 0;
   return (size_t)(threads / 32) * kTailBytesPerWarp;
 }
@@ -749,23 +782,20 @@ int mcv_run_chain(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
       launch_ms<double>(ctx, chain, ncount, first, seed, launch, s,
                         launch && launch->variant == MCV_VARIANT_FP64_FMA);
   } else if (precision == MCV_FP32) {
-    if (use_regen(chain, launch)) {
+    if (use_wave(chain, launch)) {
+      launch_wave<float>(ctx, chain, ncount, first, seed, launch, s);
+    } else if (use_regen(chain, launch)) {
       int blocks, threads;
-      const bool x = is_exotic(chain);
-      // the kX kernels take no shared-memory tally copies
-      const int tw = x ? 0 : smem_tally_words(chain);
       launch_shape(
           ctx,
-          [chain, launch, x, tw](int t) {
+          [chain, launch](int t) {
             return Launchers<float>::occupancy_regen(
-                t, (size_t)tw * 8 + regen_tail_bytes(chain, launch, t), tw,
-                x);
+                t, regen_tail_bytes(chain, launch, t));
           },
           ncount, launch, &blocks, &threads);
-      Launchers<float>::regen(
-          blocks, threads, (size_t)tw * 8 + regen_tail_bytes(chain, launch,
-                                                             threads),
-          tw, x, s, *chain, ncount, first, seed, ctx->d_status);
+      Launchers<float>::regen(blocks, threads,
+                              regen_tail_bytes(chain, launch, threads), s,
+                              *chain, ncount, first, seed, ctx->d_status);
     } else {
       launch_chain<float>(ctx, 0, chain, ncount, first, seed, nullptr, 0,
                           nullptr, nullptr, launch, s);
@@ -778,6 +808,8 @@ int mcv_run_chain(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
         launch, &blocks, &threads);
     mcv_fp64_fma_chain(x, blocks, threads, s, *chain, ncount, first, seed,
                        ctx->d_status);
+  } else if (use_wave(chain, launch)) {
+    launch_wave<double>(ctx, chain, ncount, first, seed, launch, s);
   } else {
     launch_chain<double>(ctx, 0, chain, ncount, first, seed, nullptr, 0,
                          nullptr, nullptr, launch, s);
@@ -1032,8 +1064,8 @@ int mcv_backward(mcv_ctx* ctx, const mcv_chain* chain, const mcv_grad* grad,
     py = ctx->d_grad + npeaks + 1;
   }
   int blocks, threads;
-  if (precision == MCV_FP32 && use_regen(chain, launch)) {
-    // the forward's structure (regeneration, tail queue) for the replay
+  if (precision == MCV_FP32 && use_wave(chain, launch)) {
+    // regeneration and tail queue as the forward's, for the replay
     auto bytes = [chain, launch](int t) {
       return regen_tail_bytes(chain, launch, t) ? (size_t)(t / 32) *
                                                       kGradTailBytesPerWarp
@@ -1045,13 +1077,8 @@ int mcv_backward(mcv_ctx* ctx, const mcv_chain* chain, const mcv_grad* grad,
           return Launchers<float>::occupancy_grad_regen(t, bytes(t));
         },
         ncount, launch, &blocks, &threads);
-    size_t smem = bytes(threads);
-    if (smem > 48 * 1024) {
-      cudaError_t ea = Launchers<float>::allow_grad_regen_smem(smem);
-      if (ea != cudaSuccess) return cuda_fail(st, ea, "mcv_backward smem");
-    }
-    Launchers<float>::grad_regen(blocks, threads, smem, s, *chain, *grad,
-                                 ncount, first, seed, px, py,
+    Launchers<float>::grad_regen(blocks, threads, bytes(threads), s, *chain,
+                                 *grad, ncount, first, seed, px, py,
                                  ctx->d_status);
   } else if (precision == MCV_FP32) {
     launch_shape(ctx, Launchers<float>::occupancy_grad, ncount, launch,

@@ -737,22 +737,14 @@ __device__ __forceinline__ void tail_load(const uint32_t* q, int slot,
 // with its own Philox stream, as in chain_kernel, so results agree neutron
 // by neutron (up to the compiler's contraction choices).
 //
-// Shared memory: with kSmem, first `tally_words` doubles of monitor
-// tallies (MCV_COMP_SMEM_TALLY: zeroed here, added to the global tallies
-// when the block ends), then the tail queues.  Without it (the default
-// instantiation) the kernel carries none of that code.
-template <typename R, bool kX, typename Trk, bool kSmem = false>
+// Used by the kX chains and by the FP32 backward (the forward of the other
+// chains with guides: wave.cuh).
+template <typename R, bool kX, typename Trk>
 __device__ __forceinline__ void regen_body(const mcv_chain& ch, uint64_t n,
                                            uint64_t first, uint64_t seed,
-                                           int tail_queue, int tally_words,
-                                           DevStatus* st, Trk& trk) {
+                                           int tail_queue, DevStatus* st,
+                                           Trk& trk) {
   extern __shared__ __align__(16) uint32_t tail_smem[];
-  if constexpr (!kSmem) tally_words = 0;
-  double* const smt = kSmem ? (double*)tail_smem : nullptr;
-  if constexpr (kSmem) {
-    for (int i = threadIdx.x; i < tally_words; i += blockDim.x) smt[i] = 0.0;
-    __syncthreads();
-  }
   constexpr unsigned kFull = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned below = (1u << lane) - 1u;
@@ -779,8 +771,7 @@ __device__ __forceinline__ void regen_body(const mcv_chain& ch, uint64_t n,
   // per slot: the neutron and its stream (kTailWords), then the tracker's
   // per-neutron state
   constexpr int kWords = kTailWords + Trk::kQueueWords;
-  uint32_t* q = tail_smem + 2 * tally_words +
-                (threadIdx.x >> 5) * (kWords * kTailCap);
+  uint32_t* q = tail_smem + (threadIdx.x >> 5) * (kWords * kTailCap);
   uint32_t* qt = q + kTailWords * kTailCap;
   int qhead = 0, qcount = 0;  // warp-uniform
   for (;;) {
@@ -829,7 +820,7 @@ __device__ __forceinline__ void regen_body(const mcv_chain& ch, uint64_t n,
         nb = 0;
         if (inside) continue;
       } else {
-        k.overflow += run_component<R, kX>(nt, rng, cp, trk, ch, smt);
+        k.overflow += run_component<R, kX>(nt, rng, cp, trk, ch);
       }
       if (!(nt.p > 0) || kc + 1 >= nc) {
         if (m_isnan(nt.p)) k.nonfinite++;
@@ -881,30 +872,15 @@ __device__ __forceinline__ void regen_body(const mcv_chain& ch, uint64_t n,
     }
   }
   flush_counters(k, st);
-  if constexpr (kSmem) {
-    // the block's shared-memory tallies into the global ones
-    __syncthreads();
-    for (int kc = 0; kc < nc; ++kc) {
-      const mcv_component& cp = ch.comp[kc];
-      if (!(cp.flags & kFlagSmemTally) || !cp.tally) continue;
-      const int m = 3 * (int)comp_nbins(cp);
-      const double* src = smt + cp.ip[6];
-      for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const double v = src[i];
-        if (v != 0.0) atomicAdd(cp.tally + i, v);
-      }
-    }
-  }
 }
 
-template <typename R, bool kX = false, bool kSmem = false>
+template <typename R>
 __global__ void __launch_bounds__(kMaxThreads, 4)
     regen_kernel(const __grid_constant__ mcv_chain ch, uint64_t n,
                  uint64_t first, uint64_t seed, int tail_queue,
-                 int tally_words, DevStatus* st) {
+                 DevStatus* st) {
   NoTrack trk;
-  regen_body<R, kX, NoTrack, kSmem>(ch, n, first, seed, tail_queue,
-                                    tally_words, st, trk);
+  regen_body<R, true>(ch, n, first, seed, tail_queue, st, trk);
 }
 
 // The backward replay with the regeneration kernel's structure: the same
@@ -917,9 +893,13 @@ __global__ void __launch_bounds__(kMaxThreads)
                       uint64_t first, uint64_t seed, double* powder_x,
                       double* powder_y, int tail_queue, DevStatus* st) {
   GradTrack<R> trk(g, ch, powder_x, powder_y);
-  regen_body<R, false>(ch, n, first, seed, tail_queue, 0, st, trk);
+  regen_body<R, false>(ch, n, first, seed, tail_queue, st, trk);
   trk.flush(ch);
 }
+
+}  // namespace mcv
+#include "wave.cuh"
+namespace mcv {
 
 // Backward replay: neutron i of the stream `seed` again, with the gradient
 // tracker (track.cuh) in place of the tallies.
@@ -1118,15 +1098,18 @@ struct Launchers {
                     uint64_t first, uint64_t seed, const float* uni,
                     int stride, double* out_n, int* out_last, DevStatus* st);
   // smem: the tail queue's bytes (0 = no queue)
-  // smem: the tally area (tally_words doubles) and the tail queue
-  static int occupancy_regen(int threads, size_t smem, int tally_words,
-                             bool x);
-  static void regen(int blocks, int threads, size_t smem, int tally_words,
-                    bool x, cudaStream_t s, const mcv_chain& ch, uint64_t n,
-                    uint64_t first, uint64_t seed, DevStatus* st);
+  static int occupancy_regen(int threads, size_t smem);
+  static void regen(int blocks, int threads, size_t smem, cudaStream_t s,
+                    const mcv_chain& ch, uint64_t n, uint64_t first,
+                    uint64_t seed, DevStatus* st);
+  // smem: the tally area (tally_words doubles) and the warps' queues; a
+  // kernel is allowed more than 48 KB of it when its occupancy is asked for
+  static size_t wave_smem(int threads, int tally_words);
+  static int occupancy_wave(int threads, int tally_words);
+  static void wave(int blocks, int threads, int tail_min, int tally_words,
+                   cudaStream_t s, const mcv_chain& ch, uint64_t n,
+                   uint64_t first, uint64_t seed, DevStatus* st);
   static int occupancy_grad_regen(int threads, size_t smem);
-  // dynamic shared memory above 48 KB must be allowed per kernel
-  static cudaError_t allow_grad_regen_smem(size_t smem);
   static void grad_regen(int blocks, int threads, size_t smem,
                          cudaStream_t s, const mcv_chain& ch,
                          const mcv_grad& g, uint64_t n, uint64_t first,
@@ -1160,6 +1143,14 @@ inline int occupancy_of(K kernel, int threads, size_t smem) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads,
                                                 smem);
   return per_sm < 1 ? 1 : per_sm;
+}
+
+// dynamic shared memory above 48 KB must be allowed per kernel
+template <typename K>
+inline void allow_smem(K kernel, size_t smem) {
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
 }
 
 // the chain validation of the entry points (engine.cu)
@@ -1215,44 +1206,54 @@ void Launchers<R>::chain(int mode, int x, int blocks, int threads,
 #undef MCV_CHAIN_LAUNCH
 }
 
-// kX chains take no shared-memory tally copies (tally_words is 0 there)
 template <typename R>
-int Launchers<R>::occupancy_regen(int threads, size_t smem, int tally_words,
-                                  bool x) {
-  if (x) return occupancy_of(regen_kernel<R, true>, threads, smem);
-  return tally_words ? occupancy_of(regen_kernel<R, false, true>, threads,
-                                    smem)
-                     : occupancy_of(regen_kernel<R, false>, threads, smem);
+int Launchers<R>::occupancy_regen(int threads, size_t smem) {
+  return occupancy_of(regen_kernel<R>, threads, smem);
 }
 
 template <typename R>
-void Launchers<R>::regen(int blocks, int threads, size_t smem,
-                         int tally_words, bool x, cudaStream_t s,
+void Launchers<R>::regen(int blocks, int threads, size_t smem, cudaStream_t s,
                          const mcv_chain& ch, uint64_t n, uint64_t first,
                          uint64_t seed, DevStatus* st) {
-  const int queue = smem > (size_t)tally_words * 8 ? 1 : 0;
-  if (x)
-    regen_kernel<R, true><<<blocks, threads, smem, s>>>(
-        ch, n, first, seed, queue, 0, st);
-  else if (tally_words)
-    regen_kernel<R, false, true><<<blocks, threads, smem, s>>>(
-        ch, n, first, seed, queue, tally_words, st);
+  regen_kernel<R><<<blocks, threads, smem, s>>>(ch, n, first, seed,
+                                                smem > 0 ? 1 : 0, st);
+}
+
+template <typename R>
+size_t Launchers<R>::wave_smem(int threads, int tally_words) {
+  return (size_t)tally_words * 8 +
+         (size_t)(threads / 32) * wave_warp_bytes<R>();
+}
+
+template <typename R>
+int Launchers<R>::occupancy_wave(int threads, int tally_words) {
+  const size_t smem = wave_smem(threads, tally_words);
+  if (tally_words) {
+    allow_smem(wave_kernel<R, true>, smem);
+    return occupancy_of(wave_kernel<R, true>, threads, smem);
+  }
+  allow_smem(wave_kernel<R>, smem);
+  return occupancy_of(wave_kernel<R>, threads, smem);
+}
+
+template <typename R>
+void Launchers<R>::wave(int blocks, int threads, int tail_min,
+                        int tally_words, cudaStream_t s, const mcv_chain& ch,
+                        uint64_t n, uint64_t first, uint64_t seed,
+                        DevStatus* st) {
+  const size_t smem = wave_smem(threads, tally_words);
+  if (tally_words)
+    wave_kernel<R, true><<<blocks, threads, smem, s>>>(
+        ch, n, first, seed, tail_min, tally_words, st);
   else
-    regen_kernel<R, false><<<blocks, threads, smem, s>>>(
-        ch, n, first, seed, queue, 0, st);
+    wave_kernel<R><<<blocks, threads, smem, s>>>(ch, n, first, seed, tail_min,
+                                                 0, st);
 }
 
 template <typename R>
 int Launchers<R>::occupancy_grad_regen(int threads, size_t smem) {
-  if (smem > 48 * 1024) allow_grad_regen_smem(smem);
+  allow_smem(grad_regen_kernel<R>, smem);
   return occupancy_of(grad_regen_kernel<R>, threads, smem);
-}
-
-template <typename R>
-cudaError_t Launchers<R>::allow_grad_regen_smem(size_t smem) {
-  return cudaFuncSetAttribute(grad_regen_kernel<R>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem);
 }
 
 template <typename R>

@@ -550,8 +550,10 @@ def ours_arm(a, rank, world, local_rank):
     chain64f = engine.chain_for_instrument(ins64f)
     ms64f = time_chain(chain64f, ncount, a.steps, a.warmup, "float64",
                        a.seed + 1, 0, world, rank, flush, variant="fp64_fma")
+    plain = (None if any(c.is_multiplescattering for c in ins64.components)
+             else "thread")
     ms64 = time_chain(chain64, ncount, a.steps, a.warmup, "float64",
-                      a.seed + 1, 0, world, rank, flush)
+                      a.seed + 1, 0, world, rank, flush, variant=plain)
     clk = clocks.stop()
     t64 = max_over_ranks(sum(ms64) / 1e3, world)
     t64f = max_over_ranks(sum(ms64f) / 1e3, world)

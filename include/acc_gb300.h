@@ -330,20 +330,20 @@ typedef struct mcv_launch {
   int32_t threads_per_block;
   int32_t blocks;
   int32_t chunk;            /* neutrons per work item (batched launch) */
-  int32_t variant;          /* fused FP32 kernel: 0 engine's choice,
-                               1 one neutron per thread to the end of the
-                               chain, 2 path regeneration (a lane whose
-                               neutron leaves the chain starts the next one;
-                               guides advance one bounce per step; the
-                               components after the last guide run from a
-                               per-warp queue in shared memory), 3 path
-                               regeneration without that queue.
-                               FP64 mcv_run_chain: 0 the kernel that rounds
-                               every multiply and add separately (agrees
-                               with the CPU restatement operation for
-                               operation), MCV_VARIANT_FP64_FMA the same
-                               kernel with contracted multiply-adds
-                               (faster).
+  int32_t variant;          /* fused kernels: 0 engine's choice, 1 one
+                               neutron per thread to the end of the chain,
+                               2 path regeneration where the chain has a
+                               guide (a lane whose neutron leaves the chain
+                               takes another one; guides advance one bounce
+                               per step; the components after the last guide
+                               run from a per-warp queue in shared memory),
+                               3 path regeneration that does not wait for a
+                               warp of neutrons in that queue.
+                               FP64 mcv_run_chain: 0-3 round every multiply
+                               and add separately (agree with the CPU
+                               restatement operation for operation),
+                               MCV_VARIANT_FP64_FMA the one-neutron-per-
+                               thread kernel with contracted multiply-adds.
                                Chains with a multiple scatterer followed
                                by no source or sample run, in either
                                precision, the warp-synchronous tree kernel
