@@ -235,6 +235,7 @@ __device__ __forceinline__ float f_rsqrt(float x) {
 __device__ __forceinline__ float f_div(float a, float b) {
   return __fmul_rn(a, f_rcp(b));
 }
+__device__ __forceinline__ double f_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ double f_div(double a, double b) { return a / b; }
 
 // a / b from r = 1 / b (correctly rounded): one residual correction of a r

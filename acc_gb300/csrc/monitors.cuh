@@ -16,7 +16,7 @@ namespace mcv {
 // false when that plane lies in the neutron's past.
 template <typename R>
 __device__ __forceinline__ bool to_z0(const Neutron<R>& n, R& x, R& y) {
-  R dt = -n.z / n.vz;
+  R dt = f_div(-n.z, n.vz);
   x = n.x + n.vx * dt;
   y = n.y + n.vy * dt;
   if constexpr (sizeof(R) == 8) {
@@ -32,7 +32,7 @@ __device__ __forceinline__ int bin_of(R v, R lo, R hi, int nb) {
   if constexpr (sizeof(R) == 8) {
     return clampi(m_floori((v - lo) / (hi - lo) * nb), nb);
   } else {
-    return clampi(m_floori((v - lo) * (R(nb) / (hi - lo))), nb);
+    return clampi(m_floori((v - lo) * f_div(R(nb), hi - lo)), nb);
   }
 }
 
@@ -61,8 +61,8 @@ __device__ __forceinline__ void wavelength_monitor(const Neutron<R>& n,
   R x, y;
   if (!to_z0(n, x, y)) return;
   if (!(x > xmin && x < xmax && y > ymin && y < ymax)) return;
-  R v = m_sqrt(n.vx * n.vx + n.vy * n.vy + n.vz * n.vz);
-  R L = R(2 * kPi) / (v * R(kV2K));
+  R v = f_sqrt(n.vx * n.vx + n.vy * n.vy + n.vz * n.vz);
+  R L = f_div(R(2 * kPi), v * R(kV2K));
   if (!(L > Lmin && L < Lmax)) return;
   trk.tally(tl, (uint64_t)bin_of(L, Lmin, Lmax, c.ip[0]), n.p);
 }
@@ -144,15 +144,15 @@ __device__ __forceinline__ void iqe_monitor(const Neutron<R>& n,
   R angle_in = m_atan2(vx, vz) / R(kPi) * R(180.);
   R angle_out;
   if (vy != 0) {
-    R theta = m_atan(m_sqrt(vx * vx + vz * vz) / vy) / R(kPi) * R(180.);
+    R theta = m_atan(f_sqrt(vx * vx + vz * vz) / vy) / R(kPi) * R(180.);
     angle_out = vy > 0 ? R(90.) - theta : R(90.) + theta;
   } else {
     angle_out = R(0.);
   }
   if (min_in < angle_in && angle_in < max_in && min_out < angle_out &&
       angle_out < max_out) {
-    R vi = m_sqrt(Ei) * R(kSE2V);
-    R Q = m_sqrt(vx * vx + vy * vy + (vz - vi) * (vz - vi)) * R(kV2K);
+    R vi = f_sqrt(Ei) * R(kSE2V);
+    R Q = f_sqrt(vx * vx + vy * vy + (vz - vi) * (vz - vi)) * R(kV2K);
     R E = Ei - (vx * vx + vy * vy + vz * vz) * R(kVS2E);
     if (Q >= Qmin && Q < Qmax && E >= Emin && E < Emax) {
       int iQ = bin_of(Q, Qmin, Qmax, c.ip[0]), iE = bin_of(E, Emin, Emax, c.ip[1]);
@@ -176,7 +176,7 @@ __device__ __forceinline__ void theta_tof_4pi(Neutron<R>& n,
   if (t2 < 0) return;
   if (t1 < 0) t1 = t2;
   prop_dt(n, t1);
-  R rho = m_sqrt(n.x * n.x + n.y * n.y);
+  R rho = f_sqrt(n.x * n.x + n.y * n.y);
   R theta = m_atan2(rho, n.z);
   if (m_isnan(theta)) return;
   R t = n.t.val();
@@ -196,7 +196,7 @@ __device__ __forceinline__ R vcyl_exit(const Neutron<R>& n, R Rad, R H) {
   R cc = n.x * n.x + n.z * n.z - Rad * Rad;
   R k = b * b - a * cc;
   if (k < 0 || a == 0) return NaN;
-  R t = (-b + m_sqrt(k)) / a;
+  R t = f_div(-b + f_sqrt(k), a);
   if (t < 0) return NaN;
   R y = n.y + n.vy * t;
   if (!(m_fabs(y) < H / 2)) return NaN;
@@ -214,8 +214,8 @@ __device__ __forceinline__ void cyl_iqe(Neutron<R>& n, const mcv_component& c,
   if (m_isnan(t)) return;
   prop_dt(n, t);
   R vx = n.vx, vy = n.vy, vz = n.vz;
-  R vi = m_sqrt(Ei) * R(kSE2V);
-  R Q = m_sqrt(vx * vx + vy * vy + (vz - vi) * (vz - vi)) * R(kV2K);
+  R vi = f_sqrt(Ei) * R(kSE2V);
+  R Q = f_sqrt(vx * vx + vy * vy + (vz - vi) * (vz - vi)) * R(kV2K);
   R E = Ei - (vx * vx + vy * vy + vz * vz) * R(kVS2E);
   if (Q >= Qmin && Q < Qmax && E >= Emin && E < Emax) {
     int iQ = bin_of(Q, Qmin, Qmax, c.ip[0]), iE = bin_of(E, Emin, Emax, c.ip[1]);

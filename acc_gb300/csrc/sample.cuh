@@ -32,9 +32,9 @@ __device__ __forceinline__ bool isect_sphere(R x, R y, R z, R vx, R vy, R vz,
     }
   }
   if (disc < 0) return false;
-  R s = m_sqrt(disc);
-  t1 = -(r0dotv + s) / v2;
-  t2 = -(r0dotv - s) / v2;
+  R s = f_sqrt(disc);
+  t1 = f_div(-(r0dotv + s), v2);
+  t2 = f_div(-(r0dotv - s), v2);
   return true;
 }
 
@@ -62,7 +62,7 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
   if (!(k < 0 || a == 0)) {
     bool done = false;
     if (k == 0) {
-      R t = -b / a;
+      R t = f_div(-b, a);
       if (m_fabs(z + vz * t) < hh) {
         n1 = 1;
         t1 = t;
@@ -70,8 +70,8 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
       }
     }
     if (!done) {
-      R sk = m_sqrt(k);
-      R ta = (-b + sk) / a, tb = (-b - sk) / a;
+      R sk = f_sqrt(k);
+      R ta = f_div(-b + sk, a), tb = f_div(-b - sk, a);
       bool ga = m_fabs(z + vz * ta) < hh, gb = m_fabs(z + vz * tb) < hh;
       if (ga && gb) { n1 = 2; t1 = tb; t2 = ta; }
       else if (ga) { n1 = 1; t1 = ta; }
@@ -83,10 +83,10 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
   R t3 = NaN, t4 = NaN;
   if (vz != 0) {
     R r2 = Rad * Rad;
-    R ta = (hh - z) / vz;
+    R ta = f_div(hh - z, vz);
     R xa = x + vx * ta, ya = y + vy * ta;
     bool ga = xa * xa + ya * ya <= r2;
-    R tb = (-hh - z) / vz;
+    R tb = f_div(-hh - z, vz);
     R xb = x + vx * tb, yb = y + vy * tb;
     bool gb = xb * xb + yb * yb <= r2;
     if (ga && gb) {
@@ -122,7 +122,7 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
 template <typename R>
 __device__ __forceinline__ R rect_hit(R rx, R ry, R rz, R vx, R vy, R vz, R X,
                                       R Y) {
-  R t = -rz / vz;
+  R t = f_div(-rz, vz);
   R r1x = rx + vx * t, r1y = ry + vy * t;
   if (m_fabs(r1x) > X / 2 || m_fabs(r1y) > Y / 2)
     t = R(__int_as_float(0x7fc00000));
@@ -325,7 +325,8 @@ __device__ __forceinline__ Hits<R> intersect_shape_from(const mcv_component& c,
   if constexpr (sizeof(R) == 8) {
     return intersect_shape<R>(c, x, y, z, vx, vy, vz);
   } else {
-    float t0 = -(x * vx + y * vy + z * vz) / (vx * vx + vy * vy + vz * vz);
+    float t0 = f_div(-(x * vx + y * vy + z * vz),
+                     vx * vx + vy * vy + vz * vz);
     Hits<float> h = intersect_shape<float>(c, fmaf(vx, t0, x), fmaf(vy, t0, y),
                                            fmaf(vz, t0, z), vx, vy, vz);
     h.t0 += t0;
@@ -399,10 +400,10 @@ __device__ __forceinline__ void isotropic_S(Neutron<R>& n, Rng& rng) {
   R cos_t = R(rng.next()) * 2 - 1;
   R u2 = rng.next();
   if (cos_t > 1) cos_t = 1;
-  R sin_t = m_sqrt(1 - cos_t * cos_t);
+  R sin_t = f_sqrt(1 - cos_t * cos_t);
   R sin_p, cos_p;
   m_sincos_2pi(u2, &sin_p, &cos_p);
-  R vi = m_sqrt(n.vx * n.vx + n.vy * n.vy + n.vz * n.vz);
+  R vi = f_sqrt(n.vx * n.vx + n.vy * n.vy + n.vz * n.vz);
   n.vx = vi * sin_t * cos_p;
   n.vy = vi * sin_t * sin_p;
   n.vz = vi * cos_t;
@@ -877,6 +878,13 @@ __device__ __noinline__ R expr_eval(const R* __restrict__ prog, int nops,
   return sp == 1 ? st[0] : nan;
 }
 
+// An FP64 parameter holding a whole number in [1, 2^20], read on the integer
+// pipe: a conversion is an FP64-pipe instruction, 16 clocks of the SM.
+__device__ __forceinline__ int small_int(double v) {
+  const int hi = __double2hiint(v);
+  return ((hi & 0xfffff) | 0x100000) >> (20 - ((hi >> 20) - 1023));
+}
+
 // The S of makeS (acc/kernels/E_Q.py:37-98): up to max_iter draws of Q
 // uniform on [Qmin, Qmax), each rejected while E(Q) exceeds Ei or the
 // transfer is kinematically closed (cos^2 > 1); none accepted -> p = 0.
@@ -885,7 +893,7 @@ template <typename R, typename Rng>
 __device__ __forceinline__ void e_q_scatter(Neutron<R>& n, Rng& rng,
                                             const mcv_component& c) {
   const R Qmin = prm<R>(c, 10), Qmax = prm<R>(c, 11);
-  const int max_iter = (int)c.dp[12];
+  const int max_iter = small_int(c.dp[12]);
   const int nE = c.ip[4], nS = c.ip[5];
   const R* progE = sizeof(R) == 4 ? (const R*)c.ftable : (const R*)c.table;
   const R* progS = progE + 2 * nE;
@@ -895,7 +903,7 @@ __device__ __forceinline__ void e_q_scatter(Neutron<R>& n, Rng& rng,
   R Q = 0, vf = 0, kf = 0, cost = 0, cost2 = 0;
   int itr = 0;
   bool found = false;
-  if (c.dp[13] != 0.0) {
+  if ((__double_as_longlong(c.dp[13]) << 1) != 0) {  // != 0.0
     // E does not depend on Q (dp 13, set by the host): evaluated once.
     // FP64: every try draws its Q and tests the same arithmetic as below;
     // when the neutron cannot lose E at all, every one of the max_iter
@@ -1017,7 +1025,7 @@ __device__ __forceinline__ R hss_mu(const Neutron<R>& n,
                                     const mcv_component& c) {
   // calc_absorption_coeff (acc/kernels/__init__.py:156-161)
   R v = m_sqrt(n.vx * n.vx + n.vy * n.vy + n.vz * n.vz);
-  return prm<R>(c, 8) / v * 2200;
+  return f_div(prm<R>(c, 8), v) * 2200;
 }
 
 // SANS2D_ongrid's S (acc/kernels/SANS2D_ongrid.py:16-56): (Qx, Qy) drawn
@@ -1263,7 +1271,7 @@ __device__ __forceinline__ void hss(Neutron<float>& n, Rng& rng,
                                     const mcv_component& c, Trk& trk) {
   float vx = n.vx, vy = n.vy, vz = n.vz;
   float v2 = vx * vx + vy * vy + vz * vz;
-  float t0 = -(n.x * vx + n.y * vy + n.z * vz) / v2;
+  float t0 = f_div(-(n.x * vx + n.y * vy + n.z * vz), v2);
   float px = fmaf(vx, t0, n.x), py = fmaf(vy, t0, n.y), pz = fmaf(vz, t0, n.z);
   float tau_now = -t0;
   Hits<float> h = intersect_shape<float>(c, px, py, pz, vx, vy, vz);
@@ -1310,7 +1318,7 @@ __device__ __forceinline__ void hss(Neutron<float>& n, Rng& rng,
   n.z = fmaf(vz, tau_s, pz);
   n.t.add(t0);
   n.t.add(tau_s);
-  float v = sqrtf(v2);
+  float v = sqrtf(v2);  // (shares a root with hss_sigma and hss_mu)
   float dist = v * tin, fulllen = v * T;
   float sigma = hss_sigma<float, kX>(n, c);
   float mu = hss_mu<float>(n, c);

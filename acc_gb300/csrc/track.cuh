@@ -162,7 +162,7 @@ struct GradTrack {
   double acc_g[kGradGuides][3];
   double acc_mu, acc_sig;
 
-  int hss_comp = -1, sqe_nE = 0;
+  int hss_comp = -1, sqe_nE = 0, nguides = 0;
 
   // The per-neutron state above, as queue words (FP32): word w of the
   // neutron in `slot` lives at q[w * stride + slot].
@@ -217,8 +217,10 @@ struct GradTrack {
   __device__ GradTrack(const mcv_grad& grad, const mcv_chain& ch, double* px,
                        double* py)
       : g(grad), powder_x(px), powder_y(py) {
-    for (int c = ch.ncomp - 1; c >= 0; --c)
+    for (int c = ch.ncomp - 1; c >= 0; --c) {
       if (ch.comp[c].opcode == MCV_OP_HSS) hss_comp = c;
+      nguides += ch.comp[c].opcode == MCV_OP_GUIDE;
+    }
     if (hss_comp >= 0) sqe_nE = ch.comp[hss_comp].ip[5];
 #pragma unroll
     for (int s = 0; s < kGradGuides; ++s)
@@ -316,10 +318,14 @@ struct GradTrack {
     double gb = d[bin];
     if (gb == 0.0) return;
     double gp = gb * ((double)p * t.down);
+    // FP64 work is dear (2 lanes a clock and SM): the sums of guides the
+    // chain does not have are left out
 #pragma unroll
     for (int s = 0; s < kGradGuides; ++s)
+      if (s < nguides) {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) acc_g[s][k] += gp * (double)dg[s][k];
+        for (int k = 0; k < 3; ++k) acc_g[s][k] += gp * (double)dg[s][k];
+      }
     acc_mu += gp * (double)dmu;
     acc_sig += gp * (double)dsig;
     tables(gp);
