@@ -241,11 +241,36 @@ __device__ __forceinline__ double f_div(double a, double b) { return a / b; }
 // a / b from r = 1 / b (correctly rounded): one residual correction of a r
 // gives the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34,
 // 1990), so several quotients by one divisor cost three FP64 operations each
-// instead of a division's ten, with the division's result.  Finite operands
-// and quotients in the normal range.
+// instead of a division's ten, with the division's result.  For divisors and
+// quotients well inside the range of doubles; quot() divides where one might
+// not be (the exponents are tested on the integer pipe).
 __device__ __forceinline__ double div_by(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+__device__ __forceinline__ bool mid_range(double x) {  // 2^-500 < |x| < 2^500
+  return ((__double2hiint(x) >> 20 & 0x7ff) - 523u) < 1000u;
+}
+__device__ __forceinline__ double quot(double a, double b, double r) {
+  if (mid_range(a) && mid_range(b)) return div_by(a, b, r);
+  return a / b;
+}
+__device__ __forceinline__ float quot(float a, float b, float) {
+  return f_div(a, b);
+}
+__device__ __forceinline__ double recip(double b) { return 1.0 / b; }
+__device__ __forceinline__ float recip(float) { return 0.f; }  // not used
+
+// A double as a float within 2^-23 of it, on the integer pipe (a conversion
+// is an FP64-pipe instruction, 16 clocks of the SM): 0 below 2^-126,
+// infinity from 2^128 on and for NaN.
+__device__ __forceinline__ float near_float(double d) {
+  const int hi = __double2hiint(d);
+  const unsigned m = ((unsigned)hi & 0x7fffffffu);
+  unsigned w = ((m - 0x38000000u) << 3) | ((unsigned)__double2loint(d) >> 29);
+  if (m < 0x38100000u) w = 0u;
+  if (m >= 0x47f00000u) w = 0x7f800000u;
+  return __uint_as_float(w | ((unsigned)hi & 0x80000000u));
 }
 
 __device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }

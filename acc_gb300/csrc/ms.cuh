@@ -28,6 +28,10 @@ __device__ __noinline__ Hits<R> ms_hits(const mcv_component& c, R x, R y, R z,
 }
 template <typename R>
 __device__ __noinline__ int ms_locate(const mcv_component& c, R x, R y, R z) {
+  if constexpr (sizeof(R) == 8) {
+    const int l = locate_screen(c, x, y, z);
+    if (l != kOnBorder) return l;
+  }
   return locate_shape<R>(c, x, y, z);
 }
 

@@ -10,6 +10,10 @@ namespace mcv {
 constexpr double kGeomEps = 1e-10;  // acc/geometry/__init__.py:2
 enum { kOutside = 1, kOnBorder = 0, kInside = -1 };
 
+// Marks a branch that few lanes take and that is dear (FP64 in FP32 code):
+// the compiler executed these for every lane and selected the result.
+__device__ __forceinline__ void rarely() { asm volatile(""); }
+
 // ============================================================ intersections
 // cu_device_intersect_sphere (acc/geometry/arrow_intersect.py:154-168).  In
 // FP32 the discriminant v^2 R^2 - |r x v|^2 is recomputed in FP64 when it is
@@ -25,6 +29,7 @@ __device__ __forceinline__ bool isect_sphere(R x, R y, R z, R vx, R vy, R vz,
   R disc = vR2 - r0Xv2;
   if constexpr (sizeof(R) == 4) {
     if (fabsf(disc) < 1e-4f * vR2) {
+      rarely();
       double X = x, Y = y, Z = z, VX = vx, VY = vy, VZ = vz, RR = Rad;
       double CX = Y * VZ - Z * VY, CY = Z * VX - X * VZ, CZ = X * VY - Y * VX;
       double V2 = VX * VX + VY * VY + VZ * VZ;
@@ -33,9 +38,29 @@ __device__ __forceinline__ bool isect_sphere(R x, R y, R z, R vx, R vy, R vz,
   }
   if (disc < 0) return false;
   R s = f_sqrt(disc);
-  t1 = f_div(-(r0dotv + s), v2);
-  t2 = f_div(-(r0dotv - s), v2);
+  const R rv2 = recip(v2);
+  t1 = quot(-(r0dotv + s), v2, rv2);
+  t2 = quot(-(r0dotv - s), v2, rv2);
   return true;
+}
+
+// What a ray's intersections with cylinders divide by: reciprocals of
+// vx^2 + vy^2 and vz (FP64, where a division costs ten instructions of the
+// slow pipe; the two cylinders of a CSG node share them).
+template <typename R>
+struct RayInv {
+  R ra, rz;
+};
+template <typename R>
+__device__ __forceinline__ RayInv<R> ray_inv(bool wanted, R vx, R vy, R vz) {
+  RayInv<R> ri{R(0), R(0)};
+  if constexpr (sizeof(R) == 8) {
+    if (wanted) {
+      ri.ra = recip(vx * vx + vy * vy);
+      ri.rz = recip(vz);
+    }
+  }
+  return ri;
 }
 
 // intersectCylinderSide / TopBottom / cu_device_intersect_cylinder
@@ -43,13 +68,14 @@ __device__ __forceinline__ bool isect_sphere(R x, R y, R z, R vx, R vy, R vz,
 template <typename R>
 __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
                                                R vz, R Rad, R H, R& o1,
-                                               R& o2) {
+                                               R& o2, const RayInv<R>& ri) {
   const R NaN = R(__int_as_float(0x7fc00000));
   // side
   R a = vx * vx + vy * vy, b = x * vx + y * vy, c = x * x + y * y - Rad * Rad;
   R k = b * b - a * c;
   if constexpr (sizeof(R) == 4) {
     if (fabsf(k) < 1e-4f * fmaxf(b * b, fabsf(a * c))) {
+      rarely();
       double A = (double)vx * vx + (double)vy * vy;
       double B = (double)x * vx + (double)y * vy;
       double C = (double)x * x + (double)y * y - (double)Rad * Rad;
@@ -62,7 +88,7 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
   if (!(k < 0 || a == 0)) {
     bool done = false;
     if (k == 0) {
-      R t = f_div(-b, a);
+      R t = quot(-b, a, ri.ra);
       if (m_fabs(z + vz * t) < hh) {
         n1 = 1;
         t1 = t;
@@ -71,7 +97,7 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
     }
     if (!done) {
       R sk = f_sqrt(k);
-      R ta = f_div(-b + sk, a), tb = f_div(-b - sk, a);
+      R ta = quot(-b + sk, a, ri.ra), tb = quot(-b - sk, a, ri.ra);
       bool ga = m_fabs(z + vz * ta) < hh, gb = m_fabs(z + vz * tb) < hh;
       if (ga && gb) { n1 = 2; t1 = tb; t2 = ta; }
       else if (ga) { n1 = 1; t1 = ta; }
@@ -83,10 +109,10 @@ __device__ __forceinline__ bool isect_cylinder(R x, R y, R z, R vx, R vy,
   R t3 = NaN, t4 = NaN;
   if (vz != 0) {
     R r2 = Rad * Rad;
-    R ta = f_div(hh - z, vz);
+    R ta = quot(hh - z, vz, ri.rz);
     R xa = x + vx * ta, ya = y + vy * ta;
     bool ga = xa * xa + ya * ya <= r2;
-    R tb = f_div(-hh - z, vz);
+    R tb = quot(-hh - z, vz, ri.rz);
     R xb = x + vx * tb, yb = y + vy * tb;
     bool gb = xb * xb + yb * yb <= r2;
     if (ga && gb) {
@@ -164,7 +190,8 @@ __device__ __forceinline__ bool isect_box(R x, R y, R z, R vx, R vy, R vz,
 template <typename R>
 __device__ __forceinline__ bool isect_prim(int kind, const mcv_component& c,
                                            int base, R x, R y, R z, R vx,
-                                           R vy, R vz, R& t1, R& t2) {
+                                           R vy, R vz, R& t1, R& t2,
+                                           const RayInv<R>& ri) {
   // the render wrappers (arrow_intersect.py:47-86) report no hit when t1
   // is NaN
   bool ok = false;
@@ -172,7 +199,7 @@ __device__ __forceinline__ bool isect_prim(int kind, const mcv_component& c,
     ok = isect_sphere<R>(x, y, z, vx, vy, vz, prm<R>(c, base), t1, t2);
   else if (kind == MCV_SHAPE_CYLINDER)
     ok = isect_cylinder<R>(x, y, z, vx, vy, vz, prm<R>(c, base),
-                           prm<R>(c, base + 1), t1, t2);
+                           prm<R>(c, base + 1), t1, t2, ri);
   else if (kind == MCV_SHAPE_BOX)
     ok = isect_box<R>(x, y, z, vx, vy, vz, prm<R>(c, base),
                       prm<R>(c, base + 1), prm<R>(c, base + 2), t1, t2);
@@ -264,6 +291,85 @@ __device__ __forceinline__ void cswap(R& a, R& b) {
   b = hi;
 }
 
+// Where (x, y, z), known to within `e`, certainly lies: kInside, kOutside, or
+// kOnBorder when that is not certain.
+__device__ __forceinline__ int locate_near(int kind, const mcv_component& c,
+                                           int base, float x, float y,
+                                           float z, float e) {
+  const float a = c.fp[base], b = c.fp[base + 1];
+  float d;
+  if (kind == MCV_SHAPE_SPHERE)
+    d = sqrtf(x * x + y * y + z * z) - a;
+  else if (kind == MCV_SHAPE_CYLINDER)
+    d = fmaxf(sqrtf(x * x + y * y) - a, fabsf(z) - 0.5f * b);
+  else if (kind == MCV_SHAPE_BOX)
+    d = fmaxf(fmaxf(fabsf(x) - 0.5f * a, fabsf(y) - 0.5f * b),
+              fabsf(z) - 0.5f * c.fp[base + 2]);
+  else
+    return kOnBorder;
+  return d > e ? kOutside : (d < -e ? kInside : kOnBorder);
+}
+__device__ __forceinline__ float shape_scale(const mcv_component& c) {
+  float s = fabsf(c.fp[0]) + fabsf(c.fp[1]) + fabsf(c.fp[2]);
+  if (c.ip[0] != MCV_CSG_PRIMITIVE)
+    s += fabsf(c.fp[4]) + fabsf(c.fp[5]) + fabsf(c.fp[6]);
+  return s;
+}
+
+// FP64 locations are settled in FP32 where a point is certainly far from the
+// surfaces (1e-5 of the coordinates and sizes, against roundings of a few
+// 1e-7): locate_screen gives a point's location in the shape, or kOnBorder
+// when the FP64 tests have to be made.
+__device__ __forceinline__ int locate_screen(const mcv_component& c, double x,
+                                             double y, double z) {
+  const float fx = near_float(x), fy = near_float(y), fz = near_float(z);
+  const float e =
+      1e-5f * (fabsf(fx) + fabsf(fy) + fabsf(fz) + shape_scale(c));
+  const int l1 = locate_near(c.ip[2], c, 0, fx, fy, fz, e);
+  const int op = c.ip[0];
+  if (op == MCV_CSG_PRIMITIVE) return l1;
+  const int l2 = locate_near(c.ip[3], c, 4, fx, fy, fz, e);
+  if (op == MCV_CSG_UNION) {
+    if (l1 == kInside || l2 == kInside) return kInside;
+    return l1 == kOutside && l2 == kOutside ? kOutside : kOnBorder;
+  }
+  const int in2 = op == MCV_CSG_DIFFERENCE ? kOutside : kInside;
+  const int out2 = op == MCV_CSG_DIFFERENCE ? kInside : kOutside;
+  if (l1 == kOutside || l2 == out2) return kOutside;
+  return l1 == kInside && l2 == in2 ? kInside : kOnBorder;
+}
+
+// Whether the hit at time t on operand 1 (`first`) or 2 of a CSG node is on
+// the node's border.  A hit on a sphere or cylinder lies on its own operand's
+// border (to far within locate's 1e-10), so the other operand decides, in
+// FP32 where its surface is certainly far away; FP64 otherwise, for anything
+// not finite, and for a hit on a box, whose locate has no tolerance inwards.
+template <typename R>
+__device__ __forceinline__ bool hit_on_border(const mcv_component& c,
+                                              bool first, R x, R y, R z, R vx,
+                                              R vy, R vz, R t) {
+  if constexpr (sizeof(R) == 8) {
+    const float ft = near_float(t);
+    const float ax = near_float(vx) * ft, ay = near_float(vy) * ft,
+                az = near_float(vz) * ft;
+    const float fx = near_float(x), fy = near_float(y), fz = near_float(z);
+    const float size = fabsf(fx) + fabsf(fy) + fabsf(fz) + fabsf(ax) +
+                       fabsf(ay) + fabsf(az) + shape_scale(c);
+    if (size < 1e3f && c.ip[first ? 2 : 3] != MCV_SHAPE_BOX) {
+      const int l = locate_near(c.ip[first ? 3 : 2], c, first ? 4 : 0,
+                                fx + ax, fy + ay, fz + az, 1e-5f * size);
+      // off the border: inside the other operand of a union and inside what
+      // a difference takes away; else outside the other operand
+      const int off = c.ip[0] == MCV_CSG_UNION ||
+                              (c.ip[0] == MCV_CSG_DIFFERENCE && first)
+                          ? kInside
+                          : kOutside;
+      if (l != kOnBorder) return l != off;
+    }
+  }
+  return locate_shape<R>(c, x + vx * t, y + vy * t, z + vz * t) == kOnBorder;
+}
+
 template <typename R>
 __device__ __forceinline__ Hits<R> intersect_shape(const mcv_component& c,
                                                    R x, R y, R z, R vx, R vy,
@@ -272,8 +378,12 @@ __device__ __forceinline__ Hits<R> intersect_shape(const mcv_component& c,
   const R inf = R(__int_as_float(0x7f800000));
   h.t0 = h.t1 = h.t2 = h.t3 = inf;
   h.n = 0;
+  const RayInv<R> ri = ray_inv<R>(
+      c.ip[2] == MCV_SHAPE_CYLINDER || (c.ip[0] != MCV_CSG_PRIMITIVE &&
+                                        c.ip[3] == MCV_SHAPE_CYLINDER),
+      vx, vy, vz);
   R a1, a2;
-  bool ha = isect_prim<R>(c.ip[2], c, 0, x, y, z, vx, vy, vz, a1, a2);
+  bool ha = isect_prim<R>(c.ip[2], c, 0, x, y, z, vx, vy, vz, a1, a2, ri);
   if (c.ip[0] == MCV_CSG_PRIMITIVE) {
     if (ha) {
       h.t0 = a1;
@@ -283,7 +393,7 @@ __device__ __forceinline__ Hits<R> intersect_shape(const mcv_component& c,
     return h;
   }
   R b1, b2;
-  bool hb = isect_prim<R>(c.ip[3], c, 4, x, y, z, vx, vy, vz, b1, b2);
+  bool hb = isect_prim<R>(c.ip[3], c, 4, x, y, z, vx, vy, vz, b1, b2, ri);
   R cand[4] = {a1, a2, b1, b2};
   bool ok[4] = {ha, ha, hb, hb};
   R s0 = inf, s1 = inf, s2 = inf, s3 = inf;
@@ -292,8 +402,7 @@ __device__ __forceinline__ Hits<R> intersect_shape(const mcv_component& c,
   for (int k = 0; k < 4; ++k) {
     if (ok[k]) {
       R t = cand[k];
-      if (locate_shape<R>(c, x + vx * t, y + vy * t, z + vz * t) ==
-          kOnBorder) {
+      if (hit_on_border<R>(c, k < 2, x, y, z, vx, vy, vz, t)) {
         if (n == 0) s0 = t;
         else if (n == 1) s1 = t;
         else if (n == 2) s2 = t;
