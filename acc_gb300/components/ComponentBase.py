@@ -36,8 +36,7 @@ def change_floattype(newtype):
 
 
 def _set(c, k, v):
-    c.dp[k] = float(v)
-    c.fp[k] = float(v)
+    c.dp[k] = c.fp[k] = float(v)
 
 
 class ComponentBase(metaclass=Curator):

@@ -729,11 +729,13 @@ int mcv_ctx_status(mcv_ctx* ctx, void* stream, uint64_t expected,
   if (!ctx) return MCV_EINVAL;
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_fail(st, e, "kernel execution");
+  // the copy into pageable memory returns once the stream's kernels and it
+  // have run; the reset is waited for too, for callers that go on elsewhere
   DevStatus h;
-  e = cudaMemcpyAsync(&h, ctx->d_status, sizeof h, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, sizeof h, s);
+  cudaError_t e =
+      cudaMemcpyAsync(&h, ctx->d_status, sizeof h, cudaMemcpyDeviceToHost, s);
+  if (e != cudaSuccess) return cuda_fail(st, e, "kernel execution");
+  e = cudaMemsetAsync(ctx->d_status, 0, sizeof h, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(st, e, "status read");
   int code = MCV_OK;

@@ -37,15 +37,20 @@ def build_chain(components, offsets=None, rotmats=None, binder=None):
     ch._components = list(components)
     ch.ncomp = nslots
     eye = np.eye(3)
+    # the hop transforms, written through array views of the struct (element
+    # by element through ctypes they took a third of a chain's building)
+    n = nat.MCV_MAX_COMPONENTS
+    views = [np.frombuffer(ch, dtype, n * w, field.offset).reshape(n, w)
+             for dtype, w, field in (
+                 (np.float64, 9, nat.mcv_chain.rot),
+                 (np.float32, 9, nat.mcv_chain.frot),
+                 (np.float64, 3, nat.mcv_chain.off),
+                 (np.float32, 3, nat.mcv_chain.foff))]
 
     def transform(slot, off, rot):
-        for k in range(9):
-            ch.rot[slot][k] = float(rot.flat[k])
-            ch.frot[slot][k] = float(rot.flat[k])
-        for k in range(3):
-            ch.off[slot][k] = float(off[k])
-            ch.foff[slot][k] = float(off[k])
-        if np.array_equal(rot, eye):
+        views[0][slot] = views[1][slot] = rot.reshape(9)
+        views[2][slot] = views[3][slot] = off
+        if (rot == eye).all():
             ch.comp[slot].flags |= nat.FLAG_IDENTITY_ROT
 
     slot = 0

@@ -92,13 +92,15 @@ def relative_transform(geometer, a, b):
 def calcTransformations(instrument):
     """Offsets (n-1, 3) and rotation matrices (n-1, 3, 3) between
     consecutive components (acc/run_script.py:141-162)."""
-    comps = instrument.components
-    offs, rots = [], []
-    for i in range(len(comps) - 1):
-        o, r = relative_transform(instrument.geometer, comps[i], comps[i + 1])
-        offs.append(o)
-        rots.append(r)
-    return np.array(offs).reshape(-1, 3), np.array(rots).reshape(-1, 3, 3)
+    g = instrument.geometer
+    placed = [(g.position(c), g.rotation(c)) for c in instrument.components]
+    n = max(len(placed) - 1, 0)
+    offs, rots = np.empty((n, 3)), np.empty((n, 3, 3))
+    for i in range(n):
+        (Pa, Ma), (Pb, Mb) = placed[i], placed[i + 1]
+        np.matmul(Ma, Pb - Pa, out=offs[i])
+        np.matmul(Mb, Ma.T, out=rots[i])
+    return offs, rots
 
 
 def applyTransformation(position, velocity, rotmat, offset):
