@@ -448,6 +448,14 @@ template <typename Occ>
 void launch_shape(const mcv_ctx* ctx, Occ occupancy, uint64_t n,
                   const mcv_launch* launch, int* blocks, int* threads) {
   int t = launch_threads(launch);
+  // Fewer neutrons than one full block an SM: blocks as small as spread them
+  // over every SM.  FP64 above all is a per-SM pipe of 2 lanes a clock: 1009
+  // neutrons of the sphere chain in 4 blocks keep 4 of 152 pipes busy.
+  const uint64_t sms = (uint64_t)ctx->sm_count;
+  if (!(launch && launch->threads_per_block > 0) && n < sms * t) {
+    const int fit = (int)((n + sms - 1) / sms + 31) / 32 * 32;
+    if (fit < t) t = fit < 32 ? 32 : fit;
+  }
   int per_sm = occupancy(t);
   uint64_t want = (n + t - 1) / t;
   uint64_t full = (uint64_t)ctx->sm_count * per_sm;
@@ -555,9 +563,20 @@ void launch_wave(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
                  cudaStream_t s) {
   int blocks, threads;
   const int tw = sizeof(R) == 4 ? smem_tally_words(chain) : 0;
-  launch_shape(
-      ctx, [tw](int t) { return Launchers<R>::occupancy_wave(t, tw); },
-      ncount, launch, &blocks, &threads);
+  if (sizeof(R) == 8) {
+    // one block an SM, whatever the count: the FP64 pipe is full with eight
+    // warps, and fewer warps fill their fronts and bounces better (guide
+    // chain: 1e5 neutrons 144 us against 211 at two blocks an SM, 1e6 308
+    // against 363, 1e7 2004 against 2037), while few neutrons spread out
+    // (1e4: 96 us against 118 in n / 256 blocks)
+    Launchers<R>::occupancy_wave(launch_threads(launch), tw);
+    threads = launch_threads(launch);
+    blocks = launch && launch->blocks > 0 ? launch->blocks : ctx->sm_count;
+  } else {
+    launch_shape(
+        ctx, [tw](int t) { return Launchers<R>::occupancy_wave(t, tw); },
+        ncount, launch, &blocks, &threads);
+  }
   Launchers<R>::wave(blocks, threads, wave_tail_min(launch), tw, s, *chain,
                      ncount, first, seed, ctx->d_status);
 }
