@@ -734,14 +734,16 @@ __device__ __forceinline__ int taper_quiet(const mcv_component& c, int seg,
 // divisions by vz and one by the opening: taper_quiet passes over those on
 // the FP32 pipe, and FP64 works on the segments where a wall may be met.
 // There it keeps the reference's operations, the walls' times compared as
-// fractions as in guide_bounce_fp64.  100 segments, 1e6 neutrons: 30.2 -> 5.45
-// ms (the pipe was 87% busy before, on 12.8 lanes).
+// fractions as in guide_bounce_fp64; a second quiet test in FP64 would cost
+// more than the bounce pass that finds no wall.  100 segments, 1e6 neutrons:
+// 30.2 -> 3.70 ms (the pipe was 87% busy before, on 12.8 lanes; with the FP64
+// quiet test 5.45 ms).
 __device__ __forceinline__ int guide_tapering_fp64(Neutron<double>& n,
                                                    const mcv_component& c) {
   const int nseg = c.ip[0];
   const double* d = static_cast<const double*>(c.table);
-  const double *w1 = d, *w2 = d + nseg, *h1 = d + 2 * nseg, *h2 = d + 3 * nseg,
-               *ww = d + 4 * nseg, *hh = d + 5 * nseg, *whalf = d + 6 * nseg,
+  const double *w1 = d, *h1 = d + 2 * nseg, *ww = d + 4 * nseg,
+               *hh = d + 5 * nseg, *whalf = d + 6 * nseg,
                *hhalf = d + 7 * nseg;
   const double l_seg = c.dp[0], R0 = c.dp[1], Qcx = c.dp[2], Qcy = c.dp[3],
                alphax = c.dp[4], alphay = c.dp[5], mx = c.dp[6], my = c.dp[7],
@@ -757,19 +759,13 @@ __device__ __forceinline__ int guide_tapering_fp64(Neutron<double>& n,
   t.add(dt);
   int overflow = 0;
   for (int seg = 0; seg < nseg; ++seg) {
+    // straight on to the entrance of the first segment that is not certainly
+    // quiet, or of the last one when all are: where the segments in between
+    // would leave the neutron
+    int loud = seg;
     if (vz > 0) {
-      // straight on to the entrance of the first segment that is not
-      // certainly quiet, or of the last one when all are: where the
-      // segments in between would leave the neutron
-      const int loud = taper_quiet(c, seg, x, y, z, vx, vy, vz);
-      if (loud > seg) {
-        seg = loud < nseg ? loud : nseg - 1;
-        dt = (seg * l_seg - z) / vz;
-        x += vx * dt;
-        y += vy * dt;
-        z += vz * dt;
-        if (loud >= nseg) break;
-      }
+      loud = taper_quiet(c, seg, x, y, z, vx, vy, vz);
+      seg = loud < nseg ? loud : nseg - 1;
     }
     const double zr = seg * l_seg;
     const double w1s = __ldg(&w1[seg]), hhalfs = __ldg(&hhalf[seg]);
@@ -780,6 +776,7 @@ __device__ __forceinline__ int guide_tapering_fp64(Neutron<double>& n,
     x += vx * dt;
     y += vy * dt;
     z += vz * dt;
+    if (loud >= nseg) break;
     if (x <= -0.5 * w1s || x >= 0.5 * w1s || y <= -hhalfs || y >= hhalfs) {
       n.p = 0;
       return 0;
@@ -795,14 +792,6 @@ __device__ __forceinline__ int guide_tapering_fp64(Neutron<double>& n,
     }
     x -= (edge + 0.5 * w1s);
     const double hadj = edge + (0.5 * w1s) - 0.5 * w1s;
-    if (vz > 0) {
-      const double tex = (zr + l_seg - z) / vz;
-      if (m_fabs(x + vx * tex) < 0.5 * __ldg(&w2[seg]) &&
-          m_fabs(y + vy * tex) < 0.5 * __ldg(&h2[seg])) {
-        x += hadj;
-        continue;
-      }
-    }
     int nb;
     for (nb = 0; nb < MCV_MAX_BOUNCES; ++nb) {
       const double av = l_seg * vx, bv = wws * vz, ah = l_seg * vy,

@@ -91,18 +91,18 @@ WORKLOADS = {
         "position-divergence and PSD monitors"),
 }
 
-# Per-neutron counts of the FP32 path-regeneration kernel on this workload,
-# from one ncu --set full capture of a 1e7-neutron launch (456 blocks x 256
-# threads): executed FP32 arithmetic (2*FFMA + FADD + FMUL, thread level),
+# Per-neutron counts of the FP32 wave kernel on this workload, from one ncu
+# --set full capture of a 5e6-neutron launch (608 blocks x 256 threads):
+# executed FP32 arithmetic (2*FFMA + FADD + FMUL, thread level),
 # warp instructions issued, and the DRAM bytes of that launch (tally bins
 # touched; it does not grow with the neutron count).
 KERNEL_COUNTS = {
-    "guide_chain": {"fp32_flops_per_neutron": 169.32,
-                    "warp_inst_per_neutron": 35.23,
-                    "thread_inst_per_neutron": 823.2,
-                    "dram_bytes_per_launch": 135936,
-                    "captured_neutrons": 10_000_000,
-                    "kernel": "mcv::regen_kernel<float>",
+    "guide_chain": {"fp32_flops_per_neutron": 161.3,
+                    "warp_inst_per_neutron": 22.17,
+                    "thread_inst_per_neutron": 587.0,
+                    "dram_bytes_per_launch": 277248,
+                    "captured_neutrons": 5_000_000,
+                    "kernel": "mcv::wave_kernel<float>",
                     "traffic_note": "the tally bins, independent of the "
                                     "neutron count"},
     # the multiple-scattering tree kernel (608 blocks x 256 threads on a

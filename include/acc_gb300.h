@@ -278,8 +278,8 @@ enum {
 #define MCV_COMP_IDENTITY_ROT 1   /* rot of this hop is the identity         */
 #define MCV_COMP_AGGREGATE 2      /* monitors: always warp-aggregate tally
                                      atomics (hot bins aggregate anyway) */
-#define MCV_COMP_SMEM_TALLY 4     /* monitors: the FP32 path-regeneration
-                                     kernel adds this monitor's entries into
+#define MCV_COMP_SMEM_TALLY 4     /* monitors: the FP32 kernel of chains
+                                     with guides adds this monitor's entries into
                                      a per-block copy of its tally in shared
                                      memory and adds that copy to `tally`
                                      when the block ends; ip[6] = the copy's
