@@ -191,7 +191,7 @@ __device__ inline void wave_screen_setup(WaveScreen& s, const mcv_chain& ch) {
   s.qdead = (float)(q * (1.0 + 1e-4));
   s.on = isfinite(s.f) && isfinite(s.e_pos) && isfinite(s.e_m) &&
          isfinite(s.kx) && isfinite(s.ky) && isfinite(s.qdead) &&
-         s.qdead > 0.f && dist < 1e6 && l < 1e6;
+         s.qdead > 0.f && dist > 1e-6 && dist < 1e6 && l < 1e6;
 }
 
 // true when the neutron certainly ends at the first guide's opening or first
