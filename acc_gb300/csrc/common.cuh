@@ -241,9 +241,9 @@ __device__ __forceinline__ double f_div(double a, double b) { return a / b; }
 // a / b from r = 1 / b (correctly rounded): one residual correction of a r
 // gives the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34,
 // 1990), so several quotients by one divisor cost three FP64 operations each
-// instead of a division's ten, with the division's result.  For divisors and
-// quotients well inside the range of doubles; quot() divides where one might
-// not be (the exponents are tested on the integer pipe).
+// instead of a division's ten, with the division's result.  For operands in
+// the middle of the range of doubles, which the caller tests as quot() does
+// (zeros, infinities and NaN are outside; mid_range is integer work).
 __device__ __forceinline__ double div_by(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-b, q, a), r, q);

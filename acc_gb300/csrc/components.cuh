@@ -450,12 +450,16 @@ __device__ __forceinline__ bool guide_enter(Neutron<R>& n,
   return true;
 }
 
-// What an FP64 bounce divides by, with its reciprocals (div_by): the length
-// |n| and |n|^2 of the side (x) and top (y) mirrors' normals (l, slope), and
-// the edge width W.  A kernel that keeps them in shared memory forms them
-// once a block; without them (nullptr) a bounce divides.
+// What an FP64 bounce divides by, with its reciprocals: the length |n| and
+// |n|^2 of the side (x) and top (y) mirrors' normals (l, slope), and the edge
+// width W.  A kernel that keeps them in shared memory forms them once a
+// block; without them (nullptr) a bounce divides.  It divides too where a
+// reciprocal does not serve (`by_n`, `by_w` false, or a numerator out of the
+// middle of the range): W = 0 (a sharp edge: the quotient is infinite with the
+// sign of q - m Qc), an infinite W or m, a W whose reciprocal overflows.
 struct GuideInv {
   double n[2], rn[2], n2[2], rn2[2], rw;
+  bool by_n[2], by_w;
 };
 __device__ __forceinline__ GuideInv guide_inv(const mcv_component& c) {
   const double l = c.dp[4];
@@ -466,8 +470,10 @@ __device__ __forceinline__ GuideInv guide_inv(const mcv_component& c) {
     g.n[k] = sqrt(g.n2[k]);
     g.rn[k] = 1.0 / g.n[k];
     g.rn2[k] = 1.0 / g.n2[k];
+    g.by_n[k] = mid_range(g.n[k]) && mid_range(g.n2[k]);
   }
   g.rw = 1.0 / c.dp[9];
+  g.by_w = mid_range(c.dp[9]);
   return g;
 }
 
@@ -621,8 +627,8 @@ __device__ __forceinline__ bool guide_bounce_fp64(Neutron<double>& n,
   const bool side = i <= 2;
   const double lw = side ? ww : hh;  // the mirror's slope term
   double q = kV2K * (-2) * vdn, d = 2 * vdn;
-  if (inv) {
-    const int w = side ? 0 : 1;
+  const int w = side ? 0 : 1;
+  if (inv && inv->by_n[w] && mid_range(d)) {  // (q is 2^-9 d)
     q = div_by(q, inv->n[w], inv->rn[w]);
     d = div_by(d, inv->n2[w], inv->rn2[w]);
   } else {
@@ -641,7 +647,9 @@ __device__ __forceinline__ bool guide_bounce_fp64(Neutron<double>& n,
   // calc_reflectivity (_guide_utils.py:6-23)
   double refl = R0;
   if (q > Qc) {
-    const double e = q - m * Qc, tmp = inv ? div_by(e, W, inv->rw) : e / W;
+    const double e = q - m * Qc;
+    const double tmp = inv && inv->by_w && mid_range(e)
+                           ? div_by(e, W, inv->rw) : e / W;
     refl = 0;
     if (tmp < 10) refl = R0 * ((1 - tanh(tmp)) * (1 - alpha * (q - Qc)) / 2);
   }

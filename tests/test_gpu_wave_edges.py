@@ -1,0 +1,94 @@
+"""Guide chains away from the usual coatings, sources and launches: the wave
+kernels (csrc/wave.cuh) against the one-neutron-per-thread kernels and the
+CPU oracle on the same streams.
+
+FP64: every neutron goes through the same rounded operations in each of the
+three, so the counts are equal; sums agree within 1e-12 between the kernels
+(order of additions) and 1e-9 with the oracle, or 1e-12 of the fullest bin (the
+tanh of two libraries in the reflectivity: 1 - tanh keeps an absolute error).
+"""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from acc_gb300 import engine
+from acc_gb300.components.monitors.energy_monitor import Energy_monitor
+from acc_gb300.components.monitors.psd_monitor import PSD_monitor
+from acc_gb300.components.optics.guide import Guide
+from acc_gb300.components.sources.source_simple import Source_simple
+from acc_gb300.instrument import instrument
+from helpers import gpu_tallies, oracle_run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _engine(engine_lib):
+    torch.cuda.init()
+    yield
+
+
+def _chain(source=None, guide=None, orientation=(0, 0, 0), bins=40):
+    """Disc source -> one guide 1 m away -> PSD and energy monitor."""
+    src = dict(radius=0.05, dist=1.0, xw=0.05, yh=0.05, E0=52.5, dE=47.5)
+    src.update(source or {})
+    g = dict(w1=0.05, h1=0.05, w2=0.05, h2=0.05, l=4.0, R0=0.99, Qc=0.0219,
+             alpha=3.0, m=3.0, W=0.003)
+    g.update(guide or {})
+    ins = instrument("edges")
+    ins.append(Source_simple("src", **src), position=(0, 0, 0))
+    ins.append(Guide("g", **g), position=(0, 0, 1.0), orientation=orientation)
+    z = 1.0 + g["l"] + 1e-3
+    ins.append(PSD_monitor("psd", xmin=-0.04, xmax=0.04, ymin=-0.04,
+                           ymax=0.04, nx=bins, ny=bins, filename="p.h5"),
+               position=(0, 0, z))
+    ins.append(Energy_monitor("e", xmin=-0.04, xmax=0.04, ymin=-0.04,
+                              ymax=0.04, Emin=0.0, Emax=100.0, nchan=50,
+                              filename="e.h5"), position=(0, 0, z))
+    return ins
+
+
+def _agree(build, n, first=5):
+    """Wave, thread and oracle FP64 runs of one stream agree; returns the
+    number of neutrons in the first monitor."""
+    a, b, c = build(), build(), build()
+    sa = engine.run_instrument(a, n, seed=77, first=first,
+                               floattype="float64")
+    sb = engine.run_instrument(b, n, seed=77, first=first,
+                               floattype="float64", variant="thread")
+    ref, stats, _, _ = oracle_run(c, n, seed=77, first=first)
+    assert sa.processed == sb.processed == stats["processed"] == n
+    assert sa.nonfinite == sb.nonfinite
+    for ta, tb, tc in zip(gpu_tallies(a).values(), gpu_tallies(b).values(),
+                          ref.values()):
+        np.testing.assert_array_equal(ta[0], tb[0])
+        np.testing.assert_array_equal(ta[0], tc[0])
+        np.testing.assert_allclose(ta[1:], tb[1:], rtol=1e-12, atol=1e-300)
+        for x, y in zip(ta[1:], tc[1:]):
+            np.testing.assert_allclose(x, y, rtol=1e-9,
+                                       atol=1e-12 * y.max(initial=0.0))
+    return int(next(iter(ref.values()))[0].sum())
+
+
+# a mirror edge without width (and with one whose reciprocal overflows), of
+# unbounded width, without and with unbounded reach
+@pytest.mark.parametrize("coating", [
+    dict(W=0.0), dict(W=0.0, m=1.5, alpha=6.07), dict(W=1e-310),
+    dict(W=math.inf), dict(m=0.0), dict(m=math.inf), dict(m=1e200),
+], ids=str)
+def test_fp64_wave_kernel_divides_by_any_edge_width(coating):
+    assert _agree(lambda: _chain(guide=coating), 20_001) > 100
+
+
+# a first guide turned against the source (no screening), and one that
+# converges so much that slow neutrons have both walls of a pair ahead
+@pytest.mark.parametrize("kw", [
+    dict(orientation=(0, 0, 30)), dict(orientation=(0.2, -0.1, 0)),
+    dict(source=dict(E0=1.0, dE=0.99), guide=dict(w2=0.01, h2=0.01, l=0.3)),
+    dict(source=dict(E0=10.0, dE=9.999), guide=dict(w2=0.02, h2=0.06)),
+], ids=str)
+def test_fp64_wave_kernel_turned_and_converging_guides(kw):
+    assert _agree(lambda: _chain(**kw), 20_001) > 50
