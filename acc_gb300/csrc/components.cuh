@@ -81,10 +81,17 @@ __device__ __forceinline__ void source_simple(Neutron<R>& n, Rng& rng,
     n.vy = vs * dy;
     n.vz = vs * dist;
   } else {
-    R dist1 = m_sqrt(dx * dx + dy * dy + dist * dist), inv = 1.0 / dist1;
-    n.vx = div_by(v * dx, dist1, inv);
-    n.vy = div_by(v * dy, dist1, inv);
-    n.vz = div_by(v * dist, dist1, inv);
+    R dist1 = m_sqrt(dx * dx + dy * dy + dist * dist);
+    if (mid_range(v) && mid_range(dist1)) {
+      const R inv = 1.0 / dist1;
+      n.vx = div_by(v * dx, dist1, inv);
+      n.vy = div_by(v * dy, dist1, inv);
+      n.vz = div_by(v * dist, dist1, inv);
+    } else {  // an infinite speed, say, which has no residual
+      n.vx = v * dx / dist1;
+      n.vy = v * dy / dist1;
+      n.vz = v * dist / dist1;
+    }
   }
   n.sx = R(0);
   n.sy = R(0);

@@ -92,3 +92,19 @@ def test_fp64_wave_kernel_divides_by_any_edge_width(coating):
 ], ids=str)
 def test_fp64_wave_kernel_turned_and_converging_guides(kw):
     assert _agree(lambda: _chain(**kw), 20_001) > 50
+
+
+def test_fp64_source_divides_unbounded_speeds():
+    """A speed that is not finite divides like any other: the components of
+    the velocity are infinite with the signs of the flight, as the oracle's."""
+    def build():
+        ins = instrument("fast")
+        ins.append(Source_simple("src", radius=0.05, dist=1.0, xw=0.05,
+                                 yh=0.05, E0=math.inf, dE=0.0))
+        return ins
+
+    out, _ = engine.replay(engine.chain_for_instrument(build()), 101, seed=3,
+                           floattype="float64")
+    _, _, ref, _ = oracle_run(build(), 101, seed=3, record=True)
+    assert np.isinf(ref[:, 3:6]).all()
+    np.testing.assert_array_equal(out.cpu().numpy()[:, 3:6], ref[:, 3:6])
