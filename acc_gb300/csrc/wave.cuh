@@ -177,6 +177,14 @@ __device__ inline void wave_screen_setup(WaveScreen& s, const mcv_chain& ch) {
   if (slow || !(dist > 0) || !(oz > 0) || !(l > 0) || !(W > 0) ||
       !isfinite(a[10]) || !(a[10] > 0) || !(a[7] > 0) || !(a[8] > 0))
     return;
+  // The speed's relative error in FP32: E0 + dE (2 u - 1) keeps a few units
+  // of 2^-24 (E0 + |dE|), and the slowest neutron has E0 - |dE| of it (the
+  // wavelength likewise).  A band that reaches down so far that this exceeds
+  // a percent runs unscreened.
+  const int at = ch.comp[0].ip[1] ? 3 : 5;
+  const double mean = a[at], half = fabs(a[at + 1]);
+  const double e_v = ldexp(8.0, -24) * (fabs(mean) + half) / (mean - half);
+  if (!(e_v < 1e-2)) return;
   const double q = fmax(g[6], g[8] * g[6] + 10.0 * W);
   const double reach = fabs(a[0]) + fabs(a[1]) + fabs(a[2]) + a[7] + a[8];
   s.f = (float)(oz / dist);
@@ -188,7 +196,10 @@ __device__ inline void wave_screen_setup(WaveScreen& s, const mcv_chain& ch) {
   s.e_m = (float)(1e-5 * (l * reach / dist + fabs(g[0]) + fabs(g[1])));
   s.kx = (float)(2 * kV2K / sqrt(l * l + g[0] * g[0]));
   s.ky = (float)(2 * kV2K / sqrt(l * l + g[1] * g[1]));
-  s.qdead = (float)(q * (1.0 + 1e-4));
+  // 1e-4 for the other factors of q (a few 2^-22); e_v bounds the speed's
+  // error, a square root halves the energy's and 1 / (1 - e) of a wavelength
+  // stays below 1 + 2 e
+  s.qdead = (float)(q * (1.0 + 1e-4 + 2.0 * e_v));
   s.on = isfinite(s.f) && isfinite(s.e_pos) && isfinite(s.e_m) &&
          isfinite(s.kx) && isfinite(s.ky) && isfinite(s.qdead) &&
          s.qdead > 0.f && dist > 1e-6 && dist < 1e6 && l < 1e6;

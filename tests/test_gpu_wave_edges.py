@@ -108,3 +108,21 @@ def test_fp64_source_divides_unbounded_speeds():
     _, _, ref, _ = oracle_run(build(), 101, seed=3, record=True)
     assert np.isinf(ref[:, 3:6]).all()
     np.testing.assert_array_equal(out.cpu().numpy()[:, 3:6], ref[:, 3:6])
+
+
+# Neutrons (stream 77) of a band that reaches down to almost nothing, whose
+# first reflection is 0.05-0.4% below the mirror's reach: in FP32 the energy
+# (wavelength) of the band's low end loses up to a percent, which puts the
+# same reflection beyond it.
+@pytest.mark.parametrize("first", [1156146778, 1165478551, 1251578636,
+                                   1303006222, 1309909697, 1319045109])
+def test_fp64_screen_keeps_the_low_end_of_an_energy_band(first):
+    band = dict(E0=52.5, dE=52.49999)
+    coat = dict(Qc=1e-3, m=1.0, W=1e-5)
+    assert _agree(lambda: _chain(source=band, guide=coat), 1, first) == 1
+
+
+def test_fp64_screen_keeps_the_low_end_of_a_wavelength_band():
+    band = dict(E0=0, dE=0, Lambda0=10.0, dLambda=9.99999)
+    coat = dict(Qc=200.0, m=1.0, W=0.1, alpha=0.0)
+    assert _agree(lambda: _chain(source=band, guide=coat), 1, 330837591) == 1
