@@ -341,9 +341,13 @@ __device__ __forceinline__ int locate_screen(const mcv_component& c, double x,
 
 // Whether the hit at time t on operand 1 (`first`) or 2 of a CSG node is on
 // the node's border.  A hit on a sphere or cylinder lies on its own operand's
-// border (to far within locate's 1e-10), so the other operand decides, in
-// FP32 where its surface is certainly far away; FP64 otherwise, for anything
-// not finite, and for a hit on a box, whose locate has no tolerance inwards.
+// border to within locate's 1e-10, unless a cylinder's side is hit from far
+// away: b^2 - a c is off by some 8 u D^2 v^2 for a ray that starts D from the
+// axis (u = 2^-53), and the hit by 4 u D^2 / R.  D^2 < 1e5 R keeps that below
+// 4.4e-11.  (A sphere's is off by some 4 u D, a cap's by u D.)  Where the hit
+// is on its own border the other operand decides, in FP32 if its surface is
+// certainly far away.  FP64 otherwise, for anything not finite, and for a hit
+// on a box, whose locate has no tolerance inwards.
 template <typename R>
 __device__ __forceinline__ bool hit_on_border(const mcv_component& c,
                                               bool first, R x, R y, R z, R vx,
@@ -355,7 +359,10 @@ __device__ __forceinline__ bool hit_on_border(const mcv_component& c,
     const float fx = near_float(x), fy = near_float(y), fz = near_float(z);
     const float size = fabsf(fx) + fabsf(fy) + fabsf(fz) + fabsf(ax) +
                        fabsf(ay) + fabsf(az) + shape_scale(c);
-    if (size < 1e3f && c.ip[first ? 2 : 3] != MCV_SHAPE_BOX) {
+    const int own = c.ip[first ? 2 : 3];
+    const bool near = own != MCV_SHAPE_CYLINDER ||
+                      fx * fx + fy * fy < 1e5f * c.fp[first ? 0 : 4];
+    if (size < 1e3f && own != MCV_SHAPE_BOX && near) {
       const int l = locate_near(c.ip[first ? 3 : 2], c, first ? 4 : 0,
                                 fx + ax, fy + ay, fz + az, 1e-5f * size);
       // off the border: inside the other operand of a union and inside what

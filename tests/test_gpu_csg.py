@@ -62,3 +62,26 @@ def test_fp64_csg_hits_match_the_oracle(name, op):
         assert cnt[i] == len(ref), (i, ray)
         scale = 0.1 / np.linalg.norm(ray[3:]) + np.abs(ref).max(initial=0.0)
         assert np.abs(ts[i, :len(ref)] - ref).max(initial=0.0) <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("name", ["hollow", "thin", "spheres"])
+@pytest.mark.parametrize("op", [Difference, Union, Intersection])
+@pytest.mark.parametrize("far", [20.0, 50.0, 200.0, 500.0])
+def test_fp64_csg_hits_of_distant_rays_match_the_oracle(name, op, far):
+    """Rays from `far` metres: a cylinder's side hits miss their surface by up
+    to 4 u far^2 / R there, so from some 20 m on some of them are off the
+    border to within 1e-10, and are left out as the reference leaves them
+    out."""
+    from oracle import binding as O
+    shapes = dict(OPERANDS, thin=(Cylinder(0.004, 0.06), Cylinder(0.002, 0.07)))
+    comp = factory(op(*shapes[name]), IsotropicKernel(1.0, 1.0))("s")
+    rays = _rays(2001, 13)
+    v = rays[:, 3:]
+    rays[:, :3] -= v * (far / np.linalg.norm(v, axis=1))[:, None]
+    ts, cnt = engine.intersect(comp, rays)
+    c = comp.to_struct(HostBinder())
+    for i, ray in enumerate(rays):
+        ref = np.asarray(O.intersect(c, ray), dtype=float).reshape(-1)
+        assert cnt[i] == len(ref), (i, ray)
+        scale = np.abs(ref).max(initial=0.0)
+        assert np.abs(ts[i, :len(ref)] - ref).max(initial=0.0) <= 1e-12 * scale
