@@ -272,6 +272,13 @@ __device__ __forceinline__ float near_float(double d) {
   if (m >= 0x47f00000u) w = 0x7f800000u;
   return __uint_as_float(w | ((unsigned)hi & 0x80000000u));
 }
+// A positive double of a table as a float at most 2^-20 below it, from its
+// high word alone; 0 outside the range of normal floats.
+__device__ __forceinline__ float float_below(const double* d) {
+  const int hi = __ldg(reinterpret_cast<const int*>(d) + 1);
+  const bool in = hi > 0x38100000 && hi < 0x47f00000;
+  return __int_as_float(in ? (hi - 0x38000000) << 3 : 0);
+}
 
 __device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double m_sqrt(double x) { return sqrt(x); }

@@ -697,22 +697,25 @@ __device__ __forceinline__ int guide(Neutron<R>& n, const mcv_component& c,
 // The first segment at or after `seg` whose channel a straight forward flight
 // from (x, y, z) might leave: FP32, with a bound on every rounding (positions
 // and planes: a few 1e-7 of |x| + |slope| times the guide's length; openings:
-// 1e-6), so that each segment passed over certainly holds the flight.
+// 1e-6 and, from the doubles' high words, up to another 1e-6 narrower), so
+// that each segment passed over certainly holds the flight.
 __device__ __forceinline__ int taper_quiet(const mcv_component& c, int seg,
                                            double x, double y, double z,
                                            double vx, double vy, double vz) {
+  constexpr float kHalf = 0.4999995f;
   const int nseg = c.ip[0], blk = c.ip[1];
-  const float *w1 = c.ftable, *w2 = w1 + nseg, *h1 = w2 + nseg,
-              *h2 = h1 + nseg;
+  const double* d = static_cast<const double*>(c.table);
+  const double *w1 = d, *w2 = w1 + nseg, *h1 = w2 + nseg, *h2 = h1 + nseg;
   const int nblk = blk > 0 ? (nseg + blk - 1) / blk : 0;
-  const float* bminw = w1 + 10 * nseg;
-  const float* bminh = bminw + nblk;
-  const float l = c.fp[0], x0 = (float)x, y0 = (float)y, z0 = (float)z;
+  const double* bminw = d + 10 * nseg;
+  const double* bminh = bminw + nblk;
+  const auto half = [](const double* w) { return kHalf * float_below(w); };
+  const float l = near_float(c.dp[0]);
+  const float x0 = (float)x, y0 = (float)y, z0 = (float)z;
   const float fz = (float)vz, sx = (float)vx / fz, sy = (float)vy / fz;
   const float reach = nseg * l + fabsf(z0);
   const float ex = 1e-6f * (fabsf(x0) + fabsf(sx) * reach);
   const float ey = 1e-6f * (fabsf(y0) + fabsf(sy) * reach);
-  constexpr float kHalf = 0.4999995f;
   float za = seg * l - z0;
   float xa = fabsf(fmaf(sx, za, x0)) + ex, ya = fabsf(fmaf(sy, za, y0)) + ey;
   while (seg < nseg) {
@@ -723,7 +726,7 @@ __device__ __forceinline__ int taper_quiet(const mcv_component& c, int seg,
     const float yb = fabsf(fmaf(sy, zb, y0)) + ey;
     if (whole) {
       const int b = seg / blk;
-      const float hw = kHalf * __ldg(&bminw[b]), hh = kHalf * __ldg(&bminh[b]);
+      const float hw = half(&bminw[b]), hh = half(&bminh[b]);
       if (xa < hw && xb < hw && ya < hh && yb < hh) {
         seg = to;
         xa = xb;
@@ -734,8 +737,8 @@ __device__ __forceinline__ int taper_quiet(const mcv_component& c, int seg,
     const float zn = (seg + 1) * l - z0;
     const float xn = fabsf(fmaf(sx, zn, x0)) + ex;
     const float yn = fabsf(fmaf(sy, zn, y0)) + ey;
-    if (!(xa < kHalf * __ldg(&w1[seg]) && xn < kHalf * __ldg(&w2[seg]) &&
-          ya < kHalf * __ldg(&h1[seg]) && yn < kHalf * __ldg(&h2[seg])))
+    if (!(xa < half(&w1[seg]) && xn < half(&w2[seg]) &&
+          ya < half(&h1[seg]) && yn < half(&h2[seg])))
       break;
     ++seg;
     xa = xn;

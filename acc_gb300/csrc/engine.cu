@@ -672,6 +672,34 @@ uint64_t sum_counts(const uint64_t* counts, int nvar) {
   return t;
 }
 
+// The FP64 kernels settle points far from a sample's surfaces in FP32
+// (locate_near), from the float copies of its shape's parameters; forming
+// them in the kernel cost the hollow cylinder's multiple scattering 4%
+// (18.3 -> 19.1 ms for 3e5 neutrons).  A caller of FP64 runs need not have
+// filled fp[], so they are compared with dp[] here (the batched kernel fills
+// its staged copy itself).
+bool float_shape_ok(const mcv_component& c) {
+  if (c.opcode != MCV_OP_HSS && c.opcode != MCV_OP_HMS) return true;
+  for (int k = 0; k < 8; ++k)
+    if (c.fp[k] != (float)c.dp[k]) return false;
+  return true;
+}
+
+// The chain as the kernels of `precision` may read it: `ch`, or `*fixed`
+// filled with it and with the float copies that it lacks.
+const mcv_chain* with_float_shapes(const mcv_chain* ch, int precision,
+                                   mcv_chain* fixed) {
+  if (precision != MCV_FP64) return ch;
+  bool ok = true;
+  for (int k = 0; k < ch->ncomp; ++k) ok &= float_shape_ok(ch->comp[k]);
+  if (ok) return ch;
+  *fixed = *ch;
+  for (int k = 0; k < ch->ncomp; ++k)
+    for (int j = 0; j < 8 && !float_shape_ok(ch->comp[k]); ++j)
+      fixed->comp[k].fp[j] = (float)ch->comp[k].dp[j];
+  return fixed;
+}
+
 }  // namespace
 
 // chain validation for the other entry-point unit (noalloc.cu)
@@ -794,6 +822,8 @@ int mcv_run_chain(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
     return MCV_EINVAL;
   }
   if (ncount == 0) return st ? mcv_ctx_status(ctx, stream, 0, st) : MCV_OK;
+  mcv_chain fixed;
+  chain = with_float_shapes(chain, precision, &fixed);
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
   if (use_ms_kernel(chain, launch)) {
@@ -865,6 +895,8 @@ int mcv_replay_uniforms(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
     return MCV_EINVAL;
   }
   if (ncount == 0) return st ? mcv_ctx_status(ctx, stream, 0, st) : MCV_OK;
+  mcv_chain fixed;
+  chain = with_float_shapes(chain, precision, &fixed);
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
   int mode = uniforms ? 2 : 1;
@@ -902,6 +934,8 @@ int mcv_process_buffer(mcv_ctx* ctx, const mcv_chain* chain, void* neutrons,
     set_msg(st, MCV_EINVAL, "neutron buffer is NULL%s", "");
     return MCV_EINVAL;
   }
+  mcv_chain fixed;
+  chain = with_float_shapes(chain, precision, &fixed);
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
   int blocks, threads;
@@ -1062,6 +1096,8 @@ int mcv_backward(mcv_ctx* ctx, const mcv_chain* chain, const mcv_grad* grad,
     return MCV_EINVAL;
   }
   if (ncount == 0) return st ? mcv_ctx_status(ctx, stream, 0, st) : MCV_OK;
+  mcv_chain fixed;
+  chain = with_float_shapes(chain, precision, &fixed);
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
   double *px = nullptr, *py = nullptr;
@@ -1133,6 +1169,12 @@ int mcv_intersect(mcv_ctx* ctx, const mcv_component* hss, const double* rays,
   if (!rays || !out_ts || !out_n) {
     set_msg(st, MCV_EINVAL, "mcv_intersect: NULL buffer%s", "");
     return MCV_EINVAL;
+  }
+  mcv_component fixed;
+  if (precision == MCV_FP64 && !float_shape_ok(*hss)) {
+    fixed = *hss;
+    for (int k = 0; k < 8; ++k) fixed.fp[k] = (float)hss->dp[k];
+    hss = &fixed;
   }
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;

@@ -1064,6 +1064,12 @@ __global__ void __launch_bounds__(kMaxThreads)
       stage_chain(smem, variants + v);
       cur = v;
       __syncthreads();
+      if constexpr (sizeof(R) == 8) {
+        // the float copies of shapes that locate_near reads
+        for (int i = threadIdx.x; i < 8 * ch.ncomp; i += blockDim.x)
+          ch.comp[i / 8].fp[i % 8] = (float)ch.comp[i / 8].dp[i % 8];
+        __syncthreads();
+      }
     }
     const uint64_t a = (it - item_start[v]) * chunk;
     const uint64_t cnt = counts[v];

@@ -155,6 +155,9 @@ __device__ __noinline__ int wave_component(Neutron<R>& n, PhiloxStream& rng,
 // draws: what reaches a tally never depends on the FP32 values.
 struct WaveScreen {
   int on;
+  // the source's and the guide's parameters, and the entrance's offset, from
+  // the doubles (fp[] is the FP32 kernels')
+  float a[11], g[5], ox, oy;
   float f;           // (distance to the entrance) / (distance to the target)
   float e_pos, e_m;  // error bounds: position at the entrance, wall approach
   float kx, ky;      // q = k vz m: 2 V2K / sqrt(l^2 + slope^2)
@@ -187,6 +190,10 @@ __device__ inline void wave_screen_setup(WaveScreen& s, const mcv_chain& ch) {
   if (!(e_v < 1e-2)) return;
   const double q = fmax(g[6], g[8] * g[6] + 10.0 * W);
   const double reach = fabs(a[0]) + fabs(a[1]) + fabs(a[2]) + a[7] + a[8];
+  for (int k = 0; k < 11; ++k) s.a[k] = (float)a[k];
+  for (int k = 0; k < 5; ++k) s.g[k] = (float)g[k];
+  s.ox = (float)ch.off[1][0];
+  s.oy = (float)ch.off[1][1];
   s.f = (float)(oz / dist);
   // FP32 rounding of a few operations on values up to `reach` and the
   // hardware sine and cosine (2^-21.4) are below 2e-6 of it
@@ -202,7 +209,8 @@ __device__ inline void wave_screen_setup(WaveScreen& s, const mcv_chain& ch) {
   s.qdead = (float)(q * (1.0 + 1e-4 + 2.0 * e_v));
   s.on = isfinite(s.f) && isfinite(s.e_pos) && isfinite(s.e_m) &&
          isfinite(s.kx) && isfinite(s.ky) && isfinite(s.qdead) &&
-         s.qdead > 0.f && dist > 1e-6 && dist < 1e6 && l < 1e6;
+         s.qdead > 0.f && dist > 1e-6 && dist < 1e6 && reach < 1e6 &&
+         l < 1e6;
 }
 
 // true when the neutron certainly ends at the first guide's opening or first
@@ -210,39 +218,38 @@ __device__ inline void wave_screen_setup(WaveScreen& s, const mcv_chain& ch) {
 __device__ __forceinline__ bool wave_screen_dead(const WaveScreen& s,
                                                  const mcv_chain& ch,
                                                  PhiloxStream& rng) {
-  const mcv_component& a = ch.comp[0];
-  const mcv_component& g = ch.comp[1];
+  const int* const ip = ch.comp[0].ip;
   const float u1 = rng.next(), u2 = rng.next(), u3 = rng.next(),
               u4 = rng.next(), u5 = rng.next();
   float x, y;
-  if (a.ip[0]) {
-    x = a.fp[0] * (u1 - 0.5f);
-    y = a.fp[1] * (u2 - 0.5f);
+  if (ip[0]) {
+    x = s.a[0] * (u1 - 0.5f);
+    y = s.a[1] * (u2 - 0.5f);
   } else {
-    const float r = sqrtf(u2) * a.fp[2];
+    const float r = sqrtf(u2) * s.a[2];
     float sn, cs;
     m_sincos_2pi(u1, &sn, &cs);
     x = r * cs;
     y = r * sn;
   }
-  const float dist = a.fp[9];
-  const float dx = -a.fp[7] * (u3 - 0.5f) - x;
-  const float dy = -a.fp[8] * (u4 - 0.5f) - y;
-  const float v = a.ip[1] ? float(kK2V * 2 * kPi) /
-                                (a.fp[3] + a.fp[4] * (2.f * u5 - 1.f))
+  const float dist = s.a[9];
+  const float dx = -s.a[7] * (u3 - 0.5f) - x;
+  const float dy = -s.a[8] * (u4 - 0.5f) - y;
+  const float v = ip[1] ? float(kK2V * 2 * kPi) /
+                                (s.a[3] + s.a[4] * (2.f * u5 - 1.f))
                           : float(kSE2V) *
-                                sqrtf(a.fp[5] + a.fp[6] * (2.f * u5 - 1.f));
+                                sqrtf(s.a[5] + s.a[6] * (2.f * u5 - 1.f));
   const float vz = v * dist * rsqrtf(dx * dx + dy * dy + dist * dist);
-  const float px = fmaf(dx, s.f, x - ch.foff[1][0]);
-  const float py = fmaf(dy, s.f, y - ch.foff[1][1]);
-  const float hw = g.fp[2], hh = g.fp[3];
+  const float px = fmaf(dx, s.f, x - s.ox);
+  const float py = fmaf(dy, s.f, y - s.oy);
+  const float hw = s.g[2], hh = s.g[3];
   if (fabsf(px) > hw + s.e_pos || fabsf(py) > hh + s.e_pos) return true;
   if (!(fabsf(px) < hw - s.e_pos && fabsf(py) < hh - s.e_pos)) return false;
   // the wall ahead on each side: m is its approach over the guide's length
   // (per unit l), d its distance; it is met at the fraction d / m of l
-  const float sl = g.fp[4] / dist, lx = dx * sl, ly = dy * sl;
-  const float m[4] = {-g.fp[0] - lx, -g.fp[0] + lx, -g.fp[1] - ly,
-                      -g.fp[1] + ly};
+  const float sl = s.g[4] / dist, lx = dx * sl, ly = dy * sl;
+  const float m[4] = {-s.g[0] - lx, -s.g[0] + lx, -s.g[1] - ly,
+                      -s.g[1] + ly};
   const float d[4] = {hw + px, hw - px, hh + py, hh - py};
   float first = 1.f;  // the latest the first wall can be met; 1: the exit
   bool met = false;

@@ -8,13 +8,15 @@ three, so the counts are equal; sums agree within 1e-12 between the kernels
 tanh of two libraries in the reflectivity: 1 - tanh keeps an absolute error).
 """
 
+import ctypes
 import math
 
 import numpy as np
 import pytest
 import torch
 
-from acc_gb300 import engine
+from acc_gb300 import _native as nat
+from acc_gb300 import engine, instruments
 from acc_gb300.components.monitors.energy_monitor import Energy_monitor
 from acc_gb300.components.monitors.psd_monitor import PSD_monitor
 from acc_gb300.components.optics.guide import Guide
@@ -126,3 +128,67 @@ def test_fp64_screen_keeps_the_low_end_of_a_wavelength_band():
     band = dict(E0=0, dE=0, Lambda0=10.0, dLambda=9.99999)
     coat = dict(Qc=200.0, m=1.0, W=0.1, alpha=0.0)
     assert _agree(lambda: _chain(source=band, guide=coat), 1, 330837591) == 1
+
+
+def _strip_float_copies(ch):
+    """The chain without the float copies that the FP32 kernels read."""
+    for k in range(ch.ncomp):
+        c = ch.comp[k]
+        for j in range(len(c.fp)):
+            c.fp[j] = 0.0
+        for j in range(9):
+            ch.frot[k][j] = 0.0
+        for j in range(3):
+            ch.foff[k][j] = 0.0
+
+
+def _runs(name):
+    """Ways to run an instrument's chain in FP64, with the float copies or
+    without: the fused run, a replay, one batched variant."""
+    def fused(ch, ins):
+        engine.run_chain(ch, 3000, seed=9, floattype="float64")
+        return list(gpu_tallies(ins).values())
+
+    def replay(ch, ins):
+        out, _ = engine.replay(ch, 3000, seed=9, floattype="float64")
+        return [out.cpu().numpy()[:, 9][None]]
+
+    def batched(ch, ins):
+        arr, cnt, sd = engine._batch_arrays([ch], [3000], [9])
+        st = nat.mcv_status()
+        nat.check(nat.lib().mcv_run_batched(
+            nat.context().handle, arr, 1, cnt, sd, 64, None,
+            nat.current_stream_handle(), ctypes.byref(st)), st)
+        return list(gpu_tallies(ins).values())
+
+    runs = [fused]
+    if name != "ms_hollow_cylinder":
+        runs.append(replay)
+        if name != "tapered_guide_chain":
+            runs.append(batched)
+    return runs
+
+
+@pytest.mark.parametrize("name", ["guide_chain", "ms_hollow_cylinder",
+                                  "tapered_guide_chain", "sqe_hollow_cylinder"])
+def test_fp64_kernels_read_the_double_parameters_only(name):
+    """fp, frot, foff and a segmented guide's ftable belong to the FP32
+    kernels: an FP64 run does not depend on them."""
+    wide = torch.full((4096,), 1e3, dtype=torch.float32, device="cuda")
+    for run in _runs(name):
+        out = []
+        for strip in (False, True):
+            ins = getattr(instruments, name)()
+            ch = engine.chain_for_instrument(ins)
+            if strip:
+                _strip_float_copies(ch)
+                for k in range(ch.ncomp):
+                    c = ch.comp[k]
+                    if c.opcode == nat.OP_GUIDE_TAPERING:
+                        assert c.table_len <= wide.numel()
+                        c.ftable = wide.data_ptr()
+            out.append(run(ch, ins))
+        for a, b in zip(*out):
+            assert a[0].max() > 0
+            np.testing.assert_array_equal(a[0], b[0])
+            np.testing.assert_allclose(a[1:], b[1:], rtol=1e-12, atol=1e-300)
