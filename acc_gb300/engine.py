@@ -48,9 +48,14 @@ def build_chain(components, offsets=None, rotmats=None, binder=None):
                  (np.float32, 3, nat.mcv_chain.foff))]
 
     def transform(slot, off, rot):
-        views[0][slot] = views[1][slot] = rot.reshape(9)
-        views[2][slot] = views[3][slot] = off
-        if (rot == eye).all():
+        # three offsets and nine row-major matrix elements, in any longer or
+        # (the matrix) flatter form too
+        if off.ndim != 1 or off.size < 3 or rot.size < 9:
+            raise ValueError("a hop takes a 3-vector and a 3x3 matrix, got "
+                             f"shapes {off.shape} and {rot.shape}")
+        views[0][slot] = views[1][slot] = rot.reshape(-1)[:9]
+        views[2][slot] = views[3][slot] = off[:3]
+        if rot.shape == (3, 3) and (rot == eye).all():
             ch.comp[slot].flags |= nat.FLAG_IDENTITY_ROT
 
     slot = 0
