@@ -558,18 +558,19 @@ int wave_tail_min(const mcv_launch* launch) {
 }
 
 template <typename R>
-void launch_wave(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
-                 uint64_t first, uint64_t seed, const mcv_launch* launch,
-                 cudaStream_t s) {
+cudaError_t launch_wave(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
+                        uint64_t first, uint64_t seed,
+                        const mcv_launch* launch, cudaStream_t s) {
   int blocks, threads;
   const int tw = sizeof(R) == 4 ? smem_tally_words(chain) : 0;
+  const cudaError_t e = Launchers<R>::allow_wave(tw);
+  if (e != cudaSuccess) return e;
   if (sizeof(R) == 8) {
     // one block an SM, whatever the count: the FP64 pipe is full with eight
     // warps, and fewer warps fill their fronts and bounces better (guide
     // chain: 1e5 neutrons 144 us against 211 at two blocks an SM, 1e6 308
     // against 363, 1e7 2004 against 2037), while few neutrons spread out
     // (1e4: 96 us against 118 in n / 256 blocks)
-    Launchers<R>::occupancy_wave(launch_threads(launch), tw);
     threads = launch_threads(launch);
     blocks = launch && launch->blocks > 0 ? launch->blocks : ctx->sm_count;
   } else {
@@ -579,6 +580,7 @@ void launch_wave(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
   }
   Launchers<R>::wave(blocks, threads, wave_tail_min(launch), tw, s, *chain,
                      ncount, first, seed, ctx->d_status);
+  return cudaSuccess;
 }
 
 // Shared memory of the regeneration kernels' tail queue for blocks of
@@ -826,6 +828,7 @@ int mcv_run_chain(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
   chain = with_float_shapes(chain, precision, &fixed);
   DeviceGuard g(ctx->device);
   cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e = cudaSuccess;
   if (use_ms_kernel(chain, launch)) {
     if (precision == MCV_FP32)
       launch_ms<float>(ctx, chain, ncount, first, seed, launch, s);
@@ -834,7 +837,7 @@ int mcv_run_chain(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
                         launch && launch->variant == MCV_VARIANT_FP64_FMA);
   } else if (precision == MCV_FP32) {
     if (use_wave(chain, launch)) {
-      launch_wave<float>(ctx, chain, ncount, first, seed, launch, s);
+      e = launch_wave<float>(ctx, chain, ncount, first, seed, launch, s);
     } else if (use_regen(chain, launch)) {
       int blocks, threads;
       launch_shape(
@@ -860,12 +863,16 @@ int mcv_run_chain(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
     mcv_fp64_fma_chain(x, blocks, threads, s, *chain, ncount, first, seed,
                        ctx->d_status);
   } else if (use_wave(chain, launch)) {
-    launch_wave<double>(ctx, chain, ncount, first, seed, launch, s);
+    e = launch_wave<double>(ctx, chain, ncount, first, seed, launch, s);
   } else {
     launch_chain<double>(ctx, 0, chain, ncount, first, seed, nullptr, 0,
                          nullptr, nullptr, launch, s);
   }
-  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_fail(st, e, "mcv_run_chain smem");
+  }
+  e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(st, e, "mcv_run_chain launch");
   if (st) return mcv_ctx_status(ctx, stream, ncount, st);
   return MCV_OK;
@@ -1123,6 +1130,11 @@ int mcv_backward(mcv_ctx* ctx, const mcv_chain* chain, const mcv_grad* grad,
   int blocks, threads;
   if (precision == MCV_FP32 && use_wave(chain, launch)) {
     // regeneration and tail queue as the forward's, for the replay
+    const cudaError_t ea = Launchers<float>::allow_grad_regen();
+    if (ea != cudaSuccess) {
+      cudaGetLastError();
+      return cuda_fail(st, ea, "mcv_backward smem");
+    }
     auto bytes = [chain, launch](int t) {
       return regen_tail_bytes(chain, launch, t) ? (size_t)(t / 32) *
                                                       kGradTailBytesPerWarp

@@ -1108,13 +1108,15 @@ struct Launchers {
   static void regen(int blocks, int threads, size_t smem, cudaStream_t s,
                     const mcv_chain& ch, uint64_t n, uint64_t first,
                     uint64_t seed, DevStatus* st);
-  // smem: the tally area (tally_words doubles) and the warps' queues; a
-  // kernel is allowed more than 48 KB of it when its occupancy is asked for
+  // smem: the tally area (tally_words doubles) and the warps' queues.
+  // allow_*: once before a kernel's occupancy is asked for or it is launched
   static size_t wave_smem(int threads, int tally_words);
+  static cudaError_t allow_wave(int tally_words);
   static int occupancy_wave(int threads, int tally_words);
   static void wave(int blocks, int threads, int tail_min, int tally_words,
                    cudaStream_t s, const mcv_chain& ch, uint64_t n,
                    uint64_t first, uint64_t seed, DevStatus* st);
+  static cudaError_t allow_grad_regen();
   static int occupancy_grad_regen(int threads, size_t smem);
   static void grad_regen(int blocks, int threads, size_t smem,
                          cudaStream_t s, const mcv_chain& ch,
@@ -1151,12 +1153,14 @@ inline int occupancy_of(K kernel, int threads, size_t smem) {
   return per_sm < 1 ? 1 : per_sm;
 }
 
-// dynamic shared memory above 48 KB must be allowed per kernel
+// Dynamic shared memory above 48 KB must be allowed per kernel.  The limit is
+// the kernel's, for every thread of the process, so it is always the most
+// that any launch of it takes: a smaller one, set by another thread between
+// this thread's setting and its launch, would make that launch fail.
 template <typename K>
-inline void allow_smem(K kernel, size_t smem) {
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+inline cudaError_t allow_smem(K kernel, size_t most) {
+  return cudaFuncSetAttribute(
+      kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 // the chain validation of the entry points (engine.cu)
@@ -1232,14 +1236,17 @@ size_t Launchers<R>::wave_smem(int threads, int tally_words) {
 }
 
 template <typename R>
+cudaError_t Launchers<R>::allow_wave(int tally_words) {
+  return tally_words ? allow_smem(wave_kernel<R, true>,
+                                  wave_smem(kMaxThreads, MCV_SMEM_TALLY_MAX))
+                     : allow_smem(wave_kernel<R>, wave_smem(kMaxThreads, 0));
+}
+
+template <typename R>
 int Launchers<R>::occupancy_wave(int threads, int tally_words) {
   const size_t smem = wave_smem(threads, tally_words);
-  if (tally_words) {
-    allow_smem(wave_kernel<R, true>, smem);
-    return occupancy_of(wave_kernel<R, true>, threads, smem);
-  }
-  allow_smem(wave_kernel<R>, smem);
-  return occupancy_of(wave_kernel<R>, threads, smem);
+  return tally_words ? occupancy_of(wave_kernel<R, true>, threads, smem)
+                     : occupancy_of(wave_kernel<R>, threads, smem);
 }
 
 template <typename R>
@@ -1257,8 +1264,13 @@ void Launchers<R>::wave(int blocks, int threads, int tail_min,
 }
 
 template <typename R>
+cudaError_t Launchers<R>::allow_grad_regen() {
+  return allow_smem(grad_regen_kernel<R>,
+                    (size_t)(kMaxThreads / 32) * kGradTailBytesPerWarp);
+}
+
+template <typename R>
 int Launchers<R>::occupancy_grad_regen(int threads, size_t smem) {
-  allow_smem(grad_regen_kernel<R>, smem);
   return occupancy_of(grad_regen_kernel<R>, threads, smem);
 }
 

@@ -10,6 +10,7 @@ tanh of two libraries in the reflectivity: 1 - tanh keeps an absolute error).
 
 import ctypes
 import math
+import threading
 
 import numpy as np
 import pytest
@@ -192,3 +193,31 @@ def test_fp64_kernels_read_the_double_parameters_only(name):
             assert a[0].max() > 0
             np.testing.assert_array_equal(a[0], b[0])
             np.testing.assert_allclose(a[1:], b[1:], rtol=1e-12, atol=1e-300)
+
+
+def test_launches_of_different_block_sizes_from_two_threads():
+    """The shared memory that a kernel is allowed is a property of the kernel,
+    shared by every thread of the process: launches of another block size do
+    not take it away between a thread's request and its launch."""
+    errors = []
+
+    def work(tpb):
+        try:
+            ctx = nat.Context(torch.cuda.current_device())
+            ch = engine.chain_for_instrument(_chain())
+            L = nat.mcv_launch()
+            L.threads_per_block = tpb
+            st = nat.mcv_status()
+            for i in range(3000):
+                nat.check(nat.lib().mcv_run_chain(
+                    ctx.handle, ctypes.byref(ch), 32, 0, i, 64,
+                    ctypes.byref(L), None, ctypes.byref(st)), st)
+        except Exception as e:  # reported by the main thread
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in (256, 160)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
