@@ -451,8 +451,11 @@ void launch_shape(const mcv_ctx* ctx, Occ occupancy, uint64_t n,
   // Fewer neutrons than one full block an SM: blocks as small as spread them
   // over every SM.  FP64 above all is a per-SM pipe of 2 lanes a clock: 1009
   // neutrons of the sphere chain in 4 blocks keep 4 of 152 pipes busy.
+  // A launch that names its number of blocks keeps full ones.
   const uint64_t sms = (uint64_t)ctx->sm_count;
-  if (!(launch && launch->threads_per_block > 0) && n < sms * t) {
+  const bool free =
+      !launch || (launch->threads_per_block <= 0 && launch->blocks <= 0);
+  if (free && n < sms * t) {
     const int fit = (int)((n + sms - 1) / sms + 31) / 32 * 32;
     if (fit < t) t = fit < 32 ? 32 : fit;
   }

@@ -221,3 +221,27 @@ def test_launches_of_different_block_sizes_from_two_threads():
     for t in threads:
         t.join()
     assert not errors
+
+
+def test_a_named_grid_keeps_full_blocks():
+    """A launch that names its blocks but not their size has blocks of 256
+    threads: one block takes as long as one block of 256 (median of 9; with
+    the 32 threads that spread few neutrons over every SM, it took 3.7 times
+    as long)."""
+    ch = engine.chain_for_instrument(instruments.sphere_theta_tof())
+
+    def us(**kw):
+        times = []
+        for i in range(11):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            a.record()
+            engine.run_chain(ch, 2048, seed=i, floattype="float64", blocks=1,
+                             sync=False, **kw)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return float(np.median(times[2:]))
+
+    assert us() < 1.5 * us(threads_per_block=256)
+    engine.read_status()
