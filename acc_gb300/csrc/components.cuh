@@ -21,8 +21,10 @@ namespace mcv {
 // kWave: the wave kernels' FP32 form (wave.cuh), on the bare hardware
 // reciprocal and roots and with the roundings of its sums spelled out: the
 // compiler's choice of which product to contract into a multiply-add depends
-// on the code around an inlined call, and every kernel has to follow the same
-// neutron.  (The multiple-scattering kernel ran 2.4% slower with it.)
+// on the code around an inlined call, and the wave kernels' fronts, with and
+// without shared-memory tallies, have to follow the same neutron.  The thread,
+// batched, replay and backward kernels agree with them up to rounding.  (The
+// multiple-scattering kernel ran 2.4% slower with this form.)
 __device__ __forceinline__ float sum_squares(float a, float b, float c) {
   return fmaf(c, c, fmaf(a, a, __fmul_rn(b, b)));
 }
