@@ -82,24 +82,30 @@ def instrument(name="instrument"):
     return Instrument(name)
 
 
+def _placement(geometer, comp):
+    return geometer.position(comp), geometer.rotation(comp)
+
+
+def _hop(a, b):
+    (Pa, Ma), (Pb, Mb) = a, b
+    return Ma @ (Pb - Pa), Mb @ Ma.T
+
+
 def relative_transform(geometer, a, b):
     """(offset, rotmat) taking a neutron from a's frame to b's frame."""
-    Pa, Ma = geometer.position(a), geometer.rotation(a)
-    Pb, Mb = geometer.position(b), geometer.rotation(b)
-    return Ma @ (Pb - Pa), Mb @ Ma.T
+    return _hop(_placement(geometer, a), _placement(geometer, b))
 
 
 def calcTransformations(instrument):
     """Offsets (n-1, 3) and rotation matrices (n-1, 3, 3) between
     consecutive components (acc/run_script.py:141-162)."""
-    g = instrument.geometer
-    placed = [(g.position(c), g.rotation(c)) for c in instrument.components]
-    n = max(len(placed) - 1, 0)
+    comps = instrument.components
+    n = max(len(comps) - 1, 0)
     offs, rots = np.empty((n, 3)), np.empty((n, 3, 3))
-    for i in range(n):
-        (Pa, Ma), (Pb, Mb) = placed[i], placed[i + 1]
-        np.matmul(Ma, Pb - Pa, out=offs[i])
-        np.matmul(Mb, Ma.T, out=rots[i])
+    if n:  # (a component without a neighbour need not have been placed)
+        placed = [_placement(instrument.geometer, c) for c in comps]
+        for i in range(n):
+            offs[i], rots[i] = _hop(placed[i], placed[i + 1])
     return offs, rots
 
 

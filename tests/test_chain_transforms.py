@@ -7,7 +7,9 @@ import pytest
 
 from acc_gb300 import _native as nat
 from acc_gb300.components.optics.arm import Arm
-from acc_gb300.engine import build_chain
+from acc_gb300.engine import build_chain, chain_for_instrument
+from acc_gb300.instrument import (calcTransformations, instrument,
+                                  relative_transform)
 from acc_gb300.memory import HostBinder
 
 ROT = np.arange(1.0, 10.0).reshape(3, 3)
@@ -42,3 +44,23 @@ def test_identity_is_flagged():
 def test_refused_forms(off, rot):
     with pytest.raises((ValueError, IndexError, TypeError)):
         _hop(off, rot)
+
+
+def test_hops_of_an_instrument_are_the_relative_transforms():
+    ins = instrument("turned")
+    for k in range(3):
+        ins.append(Arm(f"a{k}"), position=(0.1 * k, -0.2, 1.0 * k),
+                   orientation=(10.0 * k, 5.0, -20.0 * k))
+    offs, rots = calcTransformations(ins)
+    assert offs.shape == (2, 3) and rots.shape == (2, 3, 3)
+    for i in range(2):
+        off, rot = relative_transform(ins.geometer, *ins.components[i:i + 2])
+        np.testing.assert_array_equal(offs[i], off)
+        np.testing.assert_array_equal(rots[i], rot)
+
+
+def test_a_single_component_needs_no_place():
+    ins = instrument("single")
+    ins.components.append(Arm("a"))
+    assert calcTransformations(ins)[0].shape == (0, 3)
+    assert chain_for_instrument(ins, HostBinder()).ncomp == 1
