@@ -21,7 +21,7 @@ SOURCES = ["engine.cu", "launch_fp32.cu", "launch_fp64.cu",
 HEADERS = ["common.cuh", "components.cuh", "sample.cuh", "monitors.cuh",
            "kernels.cuh", "wave.cuh", "ms.cuh", "track.cuh"]
 # per-source extra flags: the FP64 kernels round every multiply and add
-# separately, like the CPU restatement they are checked against; the
+# separately, as the CPU restatement does that they are checked against; the
 # contracted FP64 chain kernel lives in a namespace of its own
 EXTRA_FLAGS = {"launch_fp64.cu": ["--fmad=false"],
                "launch_fp64_fma.cu": ["-Dmcv=mcv_fma"]}

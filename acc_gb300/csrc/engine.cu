@@ -346,7 +346,7 @@ int validate_chain(const mcv_chain* ch, mcv_status* st) {
   return MCV_OK;
 }
 
-// doubles of the regeneration kernel's shared-memory tally area: up to the
+// doubles of the FP32 wave kernel's shared-memory tally area: up to the
 // end of the furthest MCV_COMP_SMEM_TALLY copy (validated above)
 int smem_tally_words(const mcv_chain* ch) {
   int words = 0;
@@ -573,7 +573,12 @@ cudaError_t launch_wave(mcv_ctx* ctx, const mcv_chain* chain, uint64_t ncount,
     // warps, and fewer warps fill their fronts and bounces better (guide
     // chain: 1e5 neutrons 144 us against 211 at two blocks an SM, 1e6 308
     // against 363, 1e7 2004 against 2037), while few neutrons spread out
-    // (1e4: 96 us against 118 in n / 256 blocks)
+    // (1e4: 96 us against 118 in n / 256 blocks).  A tail with a sample and a
+    // detector changes little: with the powder cylinder and the banked
+    // detector behind the guides 1e3 107 us against 107 at two blocks, 1e5
+    // 224 against 310, 1e6 424 against 543, 1e7 3016 against 2933; with a
+    // 15 A source, so that every neutron reaches them, 1e6 7.13 ms against
+    // 7.29
     threads = launch_threads(launch);
     blocks = launch && launch->blocks > 0 ? launch->blocks : ctx->sm_count;
   } else {

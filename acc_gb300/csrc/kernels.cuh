@@ -73,7 +73,7 @@ __device__ __forceinline__ void apply_transform(Neutron<R>& n,
 // tapered guide, multiple scatterer); the common kernels leave their code
 // out so that it weighs on neither their registers nor their instruction
 // stream (the host launches the kX kernels for such chains only).
-// `smt`: the block's shared-memory tally area (the regeneration kernel's;
+// `smt`: the block's shared-memory tally area (the FP32 wave kernel's;
 // NULL elsewhere), where monitors flagged MCV_COMP_SMEM_TALLY add.
 template <typename R, bool kX = false, typename Rng, typename Trk>
 __device__ __forceinline__ int run_component(Neutron<R>& n, Rng& rng,
@@ -990,10 +990,6 @@ __global__ void intersect_kernel(const __grid_constant__ mcv_component c,
   out_n[i] = h.n;
 }
 
-// Batched persistent launch over many instrument variants.  Blocks take
-// work items of `chunk` neutrons from a device counter (DevStatus::
-// work_next); item k belongs to the variant whose cumulative item range
-// holds k.  The block stages that variant's chain in shared memory once per
 // Copies into dst (a shared-memory mcv_chain) the parts of *src that its
 // first ncomp components use: the header, comp[0..ncomp) and the hop
 // transforms rot, off, frot, foff [0..ncomp).  The rest of dst is never
@@ -1019,6 +1015,10 @@ __device__ __forceinline__ void stage_chain(unsigned char* dst,
   }
 }
 
+// Batched persistent launch over many instrument variants.  Blocks take
+// work items of `chunk` neutrons from a device counter (DevStatus::
+// work_next); item k belongs to the variant whose cumulative item range
+// holds k.  The block stages that variant's chain in shared memory once per
 // change of variant.  Neutron i of variant v draws from Philox (seeds[v], i).
 template <typename R>
 __global__ void __launch_bounds__(kMaxThreads)

@@ -1,8 +1,12 @@
 // launch_fp64.cu -- FP64 kernel instantiations.  Compiled with
 // --fmad=false: every multiply and add rounds separately, as in the CPU
-// restatement (compiled with -ffp-contract=off), so FP64 results agree with
-// it operation for operation and differ only where the math libraries'
-// transcendental functions do.
+// restatement (compiled with -ffp-contract=off), so a neutron's arithmetic is
+// the restatement's and differs only where the math libraries' transcendental
+// functions do.  What the kernels do in another way gives the same results up
+// to a rounding: a guide's walls compared as fractions, straight flights
+// taken in one step through segments that certainly hold them, and what FP32
+// bounds settle (neutrons that certainly die at their first reflection,
+// points far from a sample's surfaces).
 #define MCV_DEFINE_LAUNCHERS
 #include "kernels.cuh"
 

@@ -14,19 +14,22 @@
 //   tail    32 neutrons that left the last guide, through the components
 //           after it (monitors, a sample, a detector), from the tail queue
 //
-// Every neutron goes through the same functions in the same order on its own
-// Philox stream as in the thread kernel.  Between the bounce loops no lane
-// holds a neutron (the loop puts back what it has in flight), so that each
-// phase has the registers to itself.
+// Every neutron goes through the same components in the same order on its own
+// Philox stream as in the thread kernel: in FP64 with the same results, in
+// FP32 with roundings of its own (kWave), which move a neutron within an ulp
+// of a bin's edge into the next bin; the FP32 backward replays with the thread
+// kernel's roundings.  Between the bounce loops no lane holds a neutron (the
+// loop puts back what it has in flight), so that each phase has the registers
+// to itself.
 //
 // Bound by instruction issue (FP32) and by the FP64 pipe.  Measured on the
 // guide chain, where nine neutrons of ten die at their first reflection and
 // 1.8% reach the monitors:
-//   FP32, 1e8 neutrons: 2.45e10 -> 4.0e10 n/s against one loop that swept
+//   FP32, 1e8 neutrons: 3.79 -> 2.16 ms against one loop that swept
 //   the chain a component at a time (35.2 warp instructions a neutron on 23
 //   lanes, two of three of them control flow, range tests of the rounded
 //   divisions and spills);
-//   FP64, 1e7 neutrons: 4.2e8 -> 4.3e9 n/s against one neutron per thread
+//   FP64, 1e7 neutrons: 23.9 -> 2.02 ms against one neutron per thread
 //   (8.6 lanes on a pipe that costs a warp instruction 16 clocks whatever
 //   its lanes), most of it from the screen below.
 #pragma once

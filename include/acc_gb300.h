@@ -146,7 +146,8 @@ enum {
 
 /*
  * Parameter slots.  Doubles go in dp[], a float copy of the same values in
- * fp[] (the FP32 kernels read fp[], the FP64 kernels dp[]), integers in ip[].
+ * fp[] (the FP32 kernels read fp[], the FP64 kernels dp[]; an FP64 call makes
+ * the floats it needs from dp[] itself), integers in ip[].
  *
  * SOURCE_SIMPLE (source_simple.py:47-112 packs the same values)
  *   ip[0]=square ip[1]=wl_distr
@@ -340,8 +341,11 @@ typedef struct mcv_launch {
                                3 path regeneration that does not wait for a
                                warp of neutrons in that queue.
                                FP64 mcv_run_chain: 0-3 round every multiply
-                               and add separately (agree with the CPU
-                               restatement operation for operation),
+                               and add separately, as the CPU restatement
+                               (a guide's walls are compared as fractions,
+                               and FP32 bounds drop neutrons that certainly
+                               die at their first reflection: the same
+                               tallies, sums to 1e-12),
                                MCV_VARIANT_FP64_FMA the one-neutron-per-
                                thread kernel with contracted multiply-adds.
                                Chains with a multiple scatterer followed
