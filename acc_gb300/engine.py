@@ -37,6 +37,7 @@ def build_chain(components, offsets=None, rotmats=None, binder=None):
     ch._components = list(components)
     ch.ncomp = nslots
     eye = np.eye(3)
+    eye9 = eye.reshape(9)
     # the hop transforms, written through array views of the struct (element
     # by element through ctypes they took a third of a chain's building)
     n = nat.MCV_MAX_COMPONENTS
@@ -48,14 +49,17 @@ def build_chain(components, offsets=None, rotmats=None, binder=None):
                  (np.float32, 3, nat.mcv_chain.foff))]
 
     def transform(slot, off, rot):
-        # three offsets and nine row-major matrix elements, in any longer or
-        # (the matrix) flatter form too
-        if off.ndim != 1 or off.size < 3 or rot.size < 9:
-            raise ValueError("a hop takes a 3-vector and a 3x3 matrix, got "
-                             f"shapes {off.shape} and {rot.shape}")
-        views[0][slot] = views[1][slot] = rot.reshape(-1)[:9]
-        views[2][slot] = views[3][slot] = off[:3]
-        if rot.shape == (3, 3) and (rot == eye).all():
+        square = rot.shape == (3, 3)
+        if not square or off.shape != (3,):
+            # three offsets and nine row-major matrix elements, in any longer
+            # or (the matrix) flatter form too
+            if off.ndim != 1 or off.size < 3 or rot.size < 9:
+                raise ValueError("a hop takes a 3-vector and a 3x3 matrix, "
+                                 f"got shapes {off.shape} and {rot.shape}")
+            off, rot = off[:3], rot.reshape(-1)[:9]
+        views[0][slot] = views[1][slot] = rot.reshape(9)
+        views[2][slot] = views[3][slot] = off
+        if square and (views[0][slot] == eye9).all():
             ch.comp[slot].flags |= nat.FLAG_IDENTITY_ROT
 
     slot = 0

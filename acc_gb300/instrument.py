@@ -82,18 +82,19 @@ def instrument(name="instrument"):
     return Instrument(name)
 
 
-def _placement(geometer, comp):
-    return geometer.position(comp), geometer.rotation(comp)
-
-
-def _hop(a, b):
-    (Pa, Ma), (Pb, Mb) = a, b
-    return Ma @ (Pb - Pa), Mb @ Ma.T
+def _hop(a, b, off, rot):
+    """Into off and rot, what takes a neutron from frame a to frame b (each a
+    position and a rotation)."""
+    np.matmul(a[1], b[0] - a[0], out=off)
+    np.matmul(b[1], a[1].T, out=rot)
+    return off, rot
 
 
 def relative_transform(geometer, a, b):
     """(offset, rotmat) taking a neutron from a's frame to b's frame."""
-    return _hop(_placement(geometer, a), _placement(geometer, b))
+    return _hop((geometer.position(a), geometer.rotation(a)),
+                (geometer.position(b), geometer.rotation(b)),
+                np.empty(3), np.empty((3, 3)))
 
 
 def calcTransformations(instrument):
@@ -103,9 +104,10 @@ def calcTransformations(instrument):
     n = max(len(comps) - 1, 0)
     offs, rots = np.empty((n, 3)), np.empty((n, 3, 3))
     if n:  # (a component without a neighbour need not have been placed)
-        placed = [_placement(instrument.geometer, c) for c in comps]
+        g = instrument.geometer
+        placed = [(g.position(c), g.rotation(c)) for c in comps]
         for i in range(n):
-            offs[i], rots[i] = _hop(placed[i], placed[i + 1])
+            _hop(placed[i], placed[i + 1], offs[i], rots[i])
     return offs, rots
 
 
