@@ -248,6 +248,12 @@ __device__ __forceinline__ double div_by(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-b, q, a), r, q);
 }
+// the division for the operands that div_by leaves, out of line: inlined
+// beside it, it cost the FP64 tree kernel 0.3%
+template <typename R>
+__device__ __noinline__ R div_out(R a, R b) {
+  return a / b;
+}
 __device__ __forceinline__ bool mid_range(double x) {  // 2^-500 < |x| < 2^500
   return ((__double2hiint(x) >> 20 & 0x7ff) - 523u) < 1000u;
 }

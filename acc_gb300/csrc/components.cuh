@@ -90,9 +90,9 @@ __device__ __forceinline__ void source_simple(Neutron<R>& n, Rng& rng,
       n.vy = div_by(v * dy, dist1, inv);
       n.vz = div_by(v * dist, dist1, inv);
     } else {  // an infinite speed, say, which has no residual
-      n.vx = v * dx / dist1;
-      n.vy = v * dy / dist1;
-      n.vz = v * dist / dist1;
+      n.vx = div_out(v * dx, dist1);
+      n.vy = div_out(v * dy, dist1);
+      n.vz = div_out(v * dist, dist1);
     }
   }
   n.sx = R(0);
@@ -640,6 +640,9 @@ __device__ __forceinline__ bool guide_bounce_fp64(Neutron<double>& n,
   if (inv && inv->by_n[w] && mid_range(d)) {  // (q is 2^-9 d)
     q = div_by(q, inv->n[w], inv->rn[w]);
     d = div_by(d, inv->n2[w], inv->rn2[w]);
+  } else if (inv) {
+    q = div_out(q, inv->n[w]);
+    d = div_out(d, inv->n2[w]);
   } else {
     const double nlen2 = l * l + lw * lw;
     q = q / sqrt(nlen2);
@@ -657,8 +660,9 @@ __device__ __forceinline__ bool guide_bounce_fp64(Neutron<double>& n,
   double refl = R0;
   if (q > Qc) {
     const double e = q - m * Qc;
-    const double tmp = inv && inv->by_w && mid_range(e)
-                           ? div_by(e, W, inv->rw) : e / W;
+    const double tmp = !inv ? e / W
+                       : inv->by_w && mid_range(e) ? div_by(e, W, inv->rw)
+                                                   : div_out(e, W);
     refl = 0;
     if (tmp < 10) refl = R0 * ((1 - tanh(tmp)) * (1 - alpha * (q - Qc)) / 2);
   }
